@@ -15,7 +15,6 @@
 // runs of a step side by side (mlstm_runs.cu).  A further kernel divides each head's o by its root mean square and
 // applies the weight and the output gate.
 #include "mlstm.cuh"
-#include "vec4.cuh"
 
 constexpr int MLSTM_VB = 16, MLSTM_DY = 16, MLSTM_THREADS = MLSTM_VB * MLSTM_DY;
 
@@ -144,52 +143,40 @@ mlstm_out_kernel(const float* __restrict__ o, const float* __restrict__ proj, in
   }
 }
 
-// The same with a head's values in registers, CH runs of four neighbouring ones a lane (V a multiple of 4, at most 128 CH), and one head
-// a warp, so that everything is requested at once: a few rows take one round trip to memory instead of one a turn (8 heads of 256:
-// 13.4 -> 4.2 us a launch, the mean of six launches of 3 rows and one of 2,787).
+// The same sums with a head's values in registers, every 32nd of them a lane as above (V at most 32 CH), and one head a warp, so that
+// everything is requested at once: a few rows take one round trip to memory instead of one a turn (8 heads of 256: 13.4 -> 4.2 us
+// a launch, the mean of six launches of 3 rows and one of 2,787).  Four neighbouring values a lane would give other sums.
 template <typename TO, int CH>
 __global__ void __launch_bounds__(128)
-mlstm_out_vec_kernel(const float* __restrict__ o, const float* __restrict__ proj, int64_t ld, int off_g,
-                     const float* __restrict__ w, float eps, TO* __restrict__ out, int64_t out_ld, int H, int V, int w_shared, int gate_mode) {
+mlstm_out_regs_kernel(const float* __restrict__ o, const float* __restrict__ proj, int64_t ld, int off_g,
+                      const float* __restrict__ w, float eps, TO* __restrict__ out, int64_t out_ld, int H, int V, int w_shared, int gate_mode) {
   const int t = blockIdx.x, lane = threadIdx.x & 31, hd = blockIdx.y * 4 + (threadIdx.x >> 5);
-  float ww[CH][4];
+  float ww[CH];
   if (hd < H)
 #pragma unroll
-    for (int c = 0; c < CH; ++c) {
-      const int v = 4 * (lane + 32 * c);
-      if (v < V) ld4(w + (w_shared ? v : hd * V + v), ww[c]);
-    }
+    for (int c = 0; c < CH; ++c)
+      if (lane + 32 * c < V) ww[c] = w[(w_shared ? 0 : hd * V) + lane + 32 * c];
   pdl_wait();
   pdl_launch_dependents();
   if (hd >= H) return;
-  const float* oo = o + ((int64_t)t * H + hd) * V;
-  const float* gg = proj + (int64_t)t * ld + off_g + hd * V;
-  float x[CH][4], g[CH][4], ss = 0.f;
-#pragma unroll
-  for (int c = 0; c < CH; ++c) {
-    const int v = 4 * (lane + 32 * c);
-    if (v < V) {
-      ld4(oo + v, x[c]);
-      if (gate_mode != 2) ld4(gg + v, g[c]);
-    }
-  }
+  const float* oo = o + ((int64_t)t * H + hd) * V + lane;
+  const float* gg = proj + (int64_t)t * ld + off_g + hd * V + lane;
+  float x[CH], g[CH], ss = 0.f;
 #pragma unroll
   for (int c = 0; c < CH; ++c)
-    if (4 * (lane + 32 * c) < V)
+    if (lane + 32 * c < V) {
+      x[c] = oo[32 * c];
+      if (gate_mode != 2) g[c] = gg[32 * c];
+    }
 #pragma unroll
-      for (int e = 0; e < 4; ++e) ss = fmaf(x[c][e], x[c][e], ss);
+  for (int c = 0; c < CH; ++c)
+    if (lane + 32 * c < V) ss = fmaf(x[c], x[c], ss);
   const float r = 1.0f / sqrtf(warp_sum(ss) / (float)V + eps);
 #pragma unroll
   for (int c = 0; c < CH; ++c) {
-    const int v = 4 * (lane + 32 * c);
-    if (v >= V) continue;
-    float y[4];
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const float gate = gate_mode == 2 ? 1.0f : (gate_mode ? g[c][e] : 1.0f) / (1.0f + expf(-g[c][e]));
-      y[e] = x[c][e] * r * ww[c][e] * gate;
-    }
-    st4(out + (int64_t)t * out_ld + hd * V + v, y);
+    if (lane + 32 * c >= V) continue;
+    const float gate = gate_mode == 2 ? 1.0f : (gate_mode ? g[c] : 1.0f) / (1.0f + expf(-g[c]));
+    out[(int64_t)t * out_ld + hd * V + lane + 32 * c] = from_f<TO>(x[c] * r * ww[c] * gate);
   }
 }
 
@@ -237,13 +224,11 @@ ME_API int me_mlstm_out(const float* o, const float* proj, int64_t ld, int off_g
   if (T == 0) return 0;
   ME_REQUIRE(T > 0 && H > 0 && V > 0 && out_ld >= (int64_t)H * V, "me_mlstm_out: bad sizes T=%d H=%d V=%d", T, H, V);
   ME_REQUIRE(gate_mode >= 0 && gate_mode <= 2 && (gate_mode == 2 || proj), "me_mlstm_out: gate mode %d", gate_mode);
-  const bool gated = gate_mode != 2;
-  if (V % 4 == 0 && V <= 512 && out_ld % 4 == 0 && on4(o, ME_F32) && on4(w, ME_F32) && on4(out, out_dtype) && (H + 3) / 4 <= 65535 &&
-      (!gated || (ld % 4 == 0 && off_g % 4 == 0 && on4(proj, ME_F32)))) {
-#define MO_CASE(CH_)                                                                                                                 \
-  me_launch(mlstm_out_vec_kernel<TO, CH_>, dim3(T, (H + 3) / 4), dim3(128), 0, stream, o, proj, ld, off_g, w, eps, (TO*)out, out_ld, H, V, \
+  if (V <= 512 && (H + 3) / 4 <= 65535) {
+#define MO_CASE(CH_)                                                                                                                  \
+  me_launch(mlstm_out_regs_kernel<TO, CH_>, dim3(T, (H + 3) / 4), dim3(128), 0, stream, o, proj, ld, off_g, w, eps, (TO*)out, out_ld, H, V, \
             w_shared, gate_mode)
-    ME_DISPATCH_DTYPE(out_dtype, TO, { if (V <= 128) MO_CASE(1); else if (V <= 256) MO_CASE(2); else MO_CASE(4); });
+    ME_DISPATCH_DTYPE(out_dtype, TO, { if (V <= 128) MO_CASE(4); else if (V <= 256) MO_CASE(8); else MO_CASE(16); });
 #undef MO_CASE
     ME_LAUNCH_CHECK("me_mlstm_out");
     return 0;

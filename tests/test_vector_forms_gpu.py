@@ -1,6 +1,7 @@
 """Kernels with a form that takes four neighbouring values at a time, against their general form, which the same call runs when one
 of its vectors does not start on 16 bytes.  Both are float32; only the order of the sums differs, so results agree to a few units
 in the last place of a sum of W terms: 32 * 2^-24 relative to the row's scale is several times what any order of these sums gives."""
+import numpy as np
 import pytest
 import torch
 
@@ -111,6 +112,31 @@ def test_mlstm_out(ops, H, V, gate, shared):
     for weight, out in zip((w, off(w)), outs):
         ops.mlstm_out(o, proj, 4, weight, 1e-5, out, H, V, shared_weight=shared, gate=gate)
     near(*outs)
+
+
+# The sum of a head's squares has one order in all forms: every 32nd value a lane, then a butterfly over the lanes.  Worked out here with numpy
+# (fused multiply-adds through 64 bits), the results are the same to the bit.  Heads of one value to beyond the form in registers.
+@pytest.mark.parametrize("H, V", [(1, 4), (2, 33), (5, 128), (8, 132), (8, 256), (3, 510), (3, 512), (2, 516)])
+@pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
+def test_mlstm_out_sums_in_one_order(ops, H, V, dt):
+    f32 = np.float32
+    rng = np.random.default_rng(H * V)
+    T = 3
+    o, w = rng.standard_normal((T, H * V), dtype=f32), rng.standard_normal(H * V, dtype=f32)
+    x = np.zeros((T, H, -(-V // 32) * 32), dtype=f32)
+    x[..., :V] = o.reshape(T, H, V)
+    s = np.zeros((T, H, 32), dtype=f32)
+    for c in range(x.shape[2] // 32):
+        v = x[..., 32 * c:32 * c + 32].astype(np.float64)
+        s = (v * v + s).astype(f32)
+    for step in (16, 8, 4, 2, 1):
+        s = s + s[..., np.arange(32) ^ step]
+    r = f32(1) / np.sqrt(s[..., :1] / f32(V) + f32(1e-5))
+    ref = torch.from_numpy((x[..., :V] * r * w.reshape(H, V)).reshape(T, H * V)).to(dt)
+    out = torch.full((T, H * V), float("nan"), device=DEV, dtype=dt)
+    o = torch.from_numpy(o).to(DEV)
+    ops.mlstm_out(o, o, 0, torch.from_numpy(w).to(DEV), 1e-5, out, H, V, gate=None)
+    assert torch.equal(out.cpu(), ref)
 
 
 @pytest.mark.parametrize("H, D, R, C, rot", [(1, 4, 4, 4, 4), (16, 64, 64, 256, 64), (5, 32, 16, 132, 8), (9, 128, 64, 512, 0), (2, 8, 12, 16, 6)])
