@@ -290,7 +290,7 @@ constexpr int LMERGE_THREADS = 128, LMERGE_KEPT = 1024;      // ranges whose wei
 __global__ void __launch_bounds__(LMERGE_THREADS)
 latent_merge_kernel(const float* __restrict__ partial, const int* __restrict__ cu_seqlens, const float* __restrict__ sink,
                     const float* __restrict__ gate, bf16* __restrict__ out, int T_total, int H, int C, int splits) {
-  __shared__ float weight_s[LMERGE_KEPT];       // a range's 2^(its maximum - M), 0 for a range without keys
+  __shared__ float weight_s[LMERGE_KEPT];       // a range's 2^(its maximum - M), -1 for a range without keys (NaN beside an infinite maximum)
   __shared__ float red[32];
   const int b = blockIdx.x, head = blockIdx.y, tid = threadIdx.x;
   const float sk = sink != nullptr ? sink[head] * LOG2E : -INFINITY;
@@ -313,9 +313,9 @@ latent_merge_kernel(const float* __restrict__ partial, const int* __restrict__ c
   for (int w = 1; w < LMERGE_THREADS / 32; ++w) M = fmaxf(M, red[w]);
   float part = 0.f;
   for (int s = tid; s < splits; s += LMERGE_THREADS) {
-    const float ms = s < LMERGE_KEPT ? weight_s[s] : base[s * stride + C], w = ms != -INFINITY ? exp2f(ms - M) : 0.f;
+    const float ms = s < LMERGE_KEPT ? weight_s[s] : base[s * stride + C], w = ms != -INFINITY ? exp2f(ms - M) : -1.f;
     if (s < LMERGE_KEPT) weight_s[s] = w;
-    if (w > 0.f) part += w * base[s * stride + C + 1];
+    if (w != -1.f) part += w * base[s * stride + C + 1];
   }
   const float Lsum = block_sum(part, red) + (sink != nullptr ? exp2f(sk - M) : 0.f);      // (its barriers also order weight_s)
   float f = Lsum > 0.f ? 1.f / Lsum : 0.f;
@@ -325,7 +325,7 @@ latent_merge_kernel(const float* __restrict__ partial, const int* __restrict__ c
 #pragma unroll 8
     for (int s = 0; s < min(splits, LMERGE_KEPT); ++s) {
       const float w = weight_s[s], o = base[s * stride + d];
-      acc = w > 0.f ? fmaf(w, o, acc) : acc;    // (a range without keys may hold anything)
+      acc = w != -1.f ? fmaf(w, o, acc) : acc;  // (a range without keys may hold anything; a NaN stays visible)
     }
     for (int s = LMERGE_KEPT; s < splits; ++s) {
       const float ms = base[s * stride + C];
