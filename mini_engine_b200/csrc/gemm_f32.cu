@@ -277,8 +277,8 @@ int launch_f32(const float* A, int64_t lda, const float* W, float* C, int64_t ld
 
 }  // namespace
 
-bool gemm_f32_takes(const float* A, int64_t lda, const float* W, int M, int K) {
-  return K % 4 == 0 && (lda % 4 == 0 || M == 1) && (uintptr_t)A % 16 == 0 && (uintptr_t)W % 16 == 0;
+bool gemm_f32_takes(const float* A, int64_t lda, const float* W, int K) {
+  return K % 4 == 0 && lda % 4 == 0 && (uintptr_t)A % 16 == 0 && (uintptr_t)W % 16 == 0;
 }
 
 int gemm_f32(const float* A, int64_t lda, const float* W, float* C, int64_t ldc, int M, int N, int K, int epi, cudaStream_t stream) {

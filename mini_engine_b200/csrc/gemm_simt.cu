@@ -88,7 +88,7 @@ ME_API int me_gemm_simt(const void* A, int a_dtype, int64_t lda, const void* W, 
   ME_REQUIRE(M > 0 && N > 0 && K > 0, "me_gemm_simt: bad sizes M=%d N=%d K=%d", M, N, K);
   ME_REQUIRE(epi == 0 || epi == 1, "me_gemm_simt: unknown epilogue %d", epi);
   ME_REQUIRE((M + BM - 1) / BM <= 65535, "me_gemm_simt: M=%d is too large", M);
-  if (a_dtype == ME_F32 && w_dtype == ME_F32 && c_dtype == ME_F32 && gemm_f32_takes((const float*)A, lda, (const float*)W, M, K)) {
+  if (a_dtype == ME_F32 && w_dtype == ME_F32 && c_dtype == ME_F32 && gemm_f32_takes((const float*)A, lda, (const float*)W, K)) {
     if (gemm_f32((const float*)A, lda, (const float*)W, (float*)C, ldc, M, N, K, epi, stream)) return 1;
     ME_LAUNCH_CHECK("me_gemm_simt (float32)");
     return 0;

@@ -60,3 +60,15 @@ def test_float32_products_of_many_tiles(ops, M, N):
         got = product(ops, x, w, epilogue)
         check(got, x, w, epilogue, 25)
         assert torch.equal(product(ops, x[5:7], w, epilogue), got[5:7])
+
+
+# rows whose distance is no multiple of four values: the general form whatever their number
+@pytest.mark.parametrize("epilogue", ["none", "silu_mul"])
+def test_a_row_alone_among_rows_at_odd_distances(ops, epilogue):
+    g = torch.Generator(DEV).manual_seed(1)
+    x = torch.randn(7, 1029, device=DEV, generator=g)[:, :1028]
+    w = torch.randn(80, 1028, device=DEV, generator=g)
+    got = product(ops, x, w, epilogue)
+    check(got, x, w, epilogue, 1028)
+    for i in (0, 4):                                                 # (row 4 starts on 16 bytes)
+        assert torch.equal(product(ops, x[i:i + 1], w, epilogue), got[i:i + 1])
