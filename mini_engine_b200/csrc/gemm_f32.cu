@@ -42,7 +42,7 @@ gemm_f32_rows_kernel(const float* __restrict__ A, int64_t lda, const float* __re
     float* dst = smem + (s % stages) * stage_floats;
     const int k0 = s * slice, pieces = min(slice, K - k0) >> 2;
     for (int r = warp; r < WR; r += 4) {
-      const float* src = W + (int64_t)(min(n0 + (r & 7), N - 1) + (r >> 3) * N) * K + k0;
+      const float* src = W + ((int64_t)min(n0 + (r & 7), N - 1) + (r >> 3) * (int64_t)N) * K + k0;
       for (int p = lane; p < pieces; p += 32) cp_async16(dst + r * stride + 4 * p, src + 4 * p, true);
     }
   };
@@ -150,7 +150,7 @@ gemm_f32_tile_kernel(const float* __restrict__ A, int64_t lda, const float* __re
     for (int i = 0; i < WROWS * 16 / TILE_THREADS; ++i) {
       const int r = lr + i * (TILE_THREADS / 16), c = EPI ? r % COLS : r, n = n0 + c;
       const bool ok = n < N && k < K;
-      cp_async16(dst + i * (TILE_THREADS / 16) * TILE_LD, ok ? W + (int64_t)(n + (EPI && r >= COLS ? N : 0)) * K + k : W, ok);
+      cp_async16(dst + i * (TILE_THREADS / 16) * TILE_LD, ok ? W + ((int64_t)n + (EPI && r >= COLS ? N : 0)) * K + k : W, ok);
     }
   };
   auto load_a = [&](int s) {
@@ -248,9 +248,12 @@ template <int TM, int TN, int EPI>
 int launch_tile(const float* A, int64_t lda, const float* W, float* C, int64_t ldc, int M, int N, int K, cudaStream_t stream) {
   static const int raised = raise_smem((const void*)gemm_f32_tile_kernel<TM, TN, EPI>, tile_smem<TM, TN>);
   if (raised) return raised;
-  constexpr int COLS = EPI ? 4 * TN : 8 * TN;
-  me_launch(gemm_f32_tile_kernel<TM, TN, EPI>, dim3((N + COLS - 1) / COLS, (M + 4 * TM - 1) / (4 * TM)), dim3(TILE_THREADS),
-            (size_t)tile_smem<TM, TN>, stream, A, lda, W, C, ldc, M, N, K);
+  constexpr int COLS = EPI ? 4 * TN : 8 * TN, MOST = 65535 * 4 * TM;       // rows of a launch: the grid's y counts tiles of rows
+  for (int m0 = 0; m0 < M; m0 += MOST) {
+    const int rows = M - m0 < MOST ? M - m0 : MOST;
+    me_launch(gemm_f32_tile_kernel<TM, TN, EPI>, dim3((N + COLS - 1) / COLS, (rows + 4 * TM - 1) / (4 * TM)), dim3(TILE_THREADS),
+              (size_t)tile_smem<TM, TN>, stream, A + (int64_t)m0 * lda, lda, W, C + (int64_t)m0 * ldc, ldc, rows, N, K);
+  }
   return 0;
 }
 
@@ -259,7 +262,7 @@ int launch_f32(const float* A, int64_t lda, const float* W, float* C, int64_t ld
   // From 5 rows on the rows kernel is bound by what it reads of shared memory, and tiles are faster where there is one for every SM
   // (8 rows: 151,936 columns of 1,024 terms 272 us against 162 in tiles, 4,096 columns 19 us either way, 1,024 columns of 2,048 terms
   // 14.4 against 20.5); 9 to 16 rows took 22.6 to 37 us where the tiles take 18.5 to 20.5.
-  const int cols = N * (EPI ? 2 : 1);
+  const int64_t cols = (int64_t)N * (EPI ? 2 : 1);
   if (M <= 4) return launch_rows<EPI, 1>(A, lda, W, C, ldc, M, N, K, stream);
   if (M <= ROWS_MAX && (cols + 31) / 32 < me_sm_count()) return launch_rows<EPI, 2>(A, lda, W, C, ldc, M, N, K, stream);
   // The tile whose share of an SM costs least: TM x TN products and, at 0.6 of a product, the TM + TN pieces read for them.  (613 rows of

@@ -72,3 +72,12 @@ def test_a_row_alone_among_rows_at_odd_distances(ops, epilogue):
     check(got, x, w, epilogue, 1028)
     for i in (0, 4):                                                 # (row 4 starts on 16 bytes)
         assert torch.equal(product(ops, x[i:i + 1], w, epilogue), got[i:i + 1])
+
+
+# more rows than tiles of rows fit the grid's y
+def test_float32_products_of_very_many_rows(ops):
+    g = torch.Generator(DEV).manual_seed(2)
+    x, w = torch.randn(65535 * 32 + 1000, 4, device=DEV, generator=g), torch.randn(3, 4, device=DEV, generator=g)
+    got = product(ops, x, w, "none")
+    check(got, x, w, "none", 1)
+    assert torch.equal(product(ops, x[-3:], w, "none"), got[-3:])
