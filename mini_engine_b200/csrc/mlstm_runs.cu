@@ -5,7 +5,7 @@
 //   S_t^T q_t = exp(b_t + m0 - m_t) S0^T q_t + sum_{s<=t} exp(b_t - b_s + gi_s - m_t) (k_s . q_t) v_s     (n_t . q_t likewise)
 //   S_L = exp(b_L + m0 - m_L) S0 + exp(b_L + x_L - m_L) U,   U = sum_s exp(gi_s - b_s - x_L) k_s v_s^T    (n_L likewise)
 // U and its sum of keys need nothing from in front of the run, so only the last line is walked in order.  All exponents are <= 0.
-// Everything is float32; the results differ from the token-by-token kernel by the order of the sums.
+// Sums of gates are 64 bits, all else is float32; the results differ from the token-by-token kernel by the order of the sums.
 //
 //   ml_state_kernel   gates, b, x and U of every run: one block = one run x one head x 64 columns
 //   ml_walk_kernel    per request, in order: states[c] <- the state in front of run c
@@ -22,7 +22,7 @@ namespace {
 constexpr int LC = MLSTM_LC, VT = 64, THREADS = 256;
 
 struct MlRun {                  // a run and head
-  float b[LC], gi[LC], x[LC];   // (beyond its last token: no further decay, gi -inf)
+  double b[LC], w[LC], x[LC];   // b_t, gi_t - b_t and its largest up to t (beyond the last token: no further decay, gi -inf)
   float m0, m1, unused[2];      // the running maximum in front of the run and behind it
 };
 
@@ -50,8 +50,9 @@ __device__ __forceinline__ void fill(float* dst, int ld_dst, int rows, int cols,
   }
 }
 
-// The first warp's work: the run's gates and their scans, two tokens a lane.
-__device__ __forceinline__ void run_gates(const MlstmArgs& a, int tok0, int L, int h, float* b_s, float* gi_s, float* x_s) {
+// The first warp's work: the run's gates and their scans, two tokens a lane.  The sums of the gates are 64 bits: they go down to -64 caps,
+// where a float is rounded to 6e-5 (cap 15), and the weights are exponentials of their differences.
+__device__ __forceinline__ void run_gates(const MlstmArgs& a, int tok0, int L, int h, double* b_s, double* w_s, double* x_s) {
   if (threadIdx.x >= 32) return;
   const int lane = threadIdx.x;
   float gf[2], gi[2];
@@ -66,26 +67,25 @@ __device__ __forceinline__ void run_gates(const MlstmArgs& a, int tok0, int L, i
       gf[e] = mlstm_log_sigmoid(mlstm_capped(row[a.off_f + h] + a.bias_f[h], a.cap));
     }
   }
-  float run = gf[0] + gf[1];
+  double run = (double)gf[0] + gf[1];
 #pragma unroll
   for (int off = 1; off < 32; off <<= 1) {
-    const float up = __shfl_up_sync(0xffffffffu, run, off);
+    const double up = __shfl_up_sync(0xffffffffu, run, off);
     if (lane >= off) run += up;
   }
-  const float b1 = run, b0 = run - gf[1];
-  const float x0 = gi[0] - b0, x1 = fmaxf(x0, gi[1] - b1);
-  float mx = x1;
+  const double b1 = run, b0 = run - gf[1], w0 = gi[0] - b0, w1 = gi[1] - b1;
+  double mx = fmax(w0, w1);
 #pragma unroll
   for (int off = 1; off < 32; off <<= 1) {
-    const float up = __shfl_up_sync(0xffffffffu, mx, off);
-    if (lane >= off) mx = fmaxf(mx, up);
+    const double up = __shfl_up_sync(0xffffffffu, mx, off);
+    if (lane >= off) mx = fmax(mx, up);
   }
-  const float before = __shfl_up_sync(0xffffffffu, mx, 1);
+  const double before = __shfl_up_sync(0xffffffffu, mx, 1);
   b_s[2 * lane] = b0;
   b_s[2 * lane + 1] = b1;
-  gi_s[2 * lane] = gi[0];
-  gi_s[2 * lane + 1] = gi[1];
-  x_s[2 * lane] = lane > 0 ? fmaxf(before, x0) : x0;
+  w_s[2 * lane] = w0;
+  w_s[2 * lane + 1] = w1;
+  x_s[2 * lane] = lane > 0 ? fmax(before, w0) : w0;
   x_s[2 * lane + 1] = mx;
 }
 
@@ -93,7 +93,8 @@ template <int VEC>
 __global__ void __launch_bounds__(THREADS)
 ml_state_kernel(MlstmArgs a, const int* __restrict__ tiles, float* __restrict__ states, float* __restrict__ key_sums, MlRun* __restrict__ runs) {
   extern __shared__ __align__(16) float smem[];
-  __shared__ float b_s[LC], gi_s[LC], x_s[LC];
+  __shared__ double b_s[LC], w_s[LC], x_s[LC];
+  __shared__ float u_s[LC];                     // a token's weight in U
   const int D = a.D, V = a.V, Dp = (D + 63) / 64 * 64, ldk = Dp + 4;
   float* Kt = smem;                             // [LC][Dp + 4]
   float* Vc = Kt + LC * ldk;                    // [LC][VT], times a token's weight
@@ -103,16 +104,19 @@ ml_state_kernel(MlstmArgs a, const int* __restrict__ tiles, float* __restrict__ 
   pdl_wait();
   pdl_launch_dependents();
   if (L <= 0) return;
-  run_gates(a, tok0, L, h, b_s, gi_s, x_s);
+  run_gates(a, tok0, L, h, b_s, w_s, x_s);
   fill<VEC>(Kt, ldk, LC, Dp, a.proj + (int64_t)tok0 * a.ld + a.off_k + (int64_t)h * D, a.ld, L, D);
   __syncthreads();
-  const float xl = x_s[LC - 1];
-  if (tid < LC && blockIdx.z == 0) {
-    MlRun& run = runs[(int64_t)blockIdx.x * a.H + h];
-    run.b[tid] = b_s[tid];
-    run.gi[tid] = gi_s[tid];
-    run.x[tid] = x_s[tid];
+  if (tid < LC) {
+    u_s[tid] = tid < L ? expf((float)(w_s[tid] - x_s[LC - 1])) : 0.f;
+    if (blockIdx.z == 0) {
+      MlRun& run = runs[(int64_t)blockIdx.x * a.H + h];
+      run.b[tid] = b_s[tid];
+      run.w[tid] = w_s[tid];
+      run.x[tid] = x_s[tid];
+    }
   }
+  __syncthreads();
   {
     const float* src = a.proj + (int64_t)tok0 * a.ld + a.off_v + (int64_t)h * V + v0;
     constexpr int per = VT / VEC;
@@ -121,9 +125,8 @@ ml_state_kernel(MlstmArgs a, const int* __restrict__ tiles, float* __restrict__ 
       const int r = i / per, c = (i - r * per) * VEC;
       float v[VEC] = {};
       if (r < L && v0 + c < V) ldv<VEC>(src + (int64_t)r * a.ld + c, v);
-      const float w = r < L ? expf(gi_s[r] - b_s[r] - xl) : 0.f;
 #pragma unroll
-      for (int j = 0; j < VEC; ++j) v[j] *= w;
+      for (int j = 0; j < VEC; ++j) v[j] *= u_s[r];
       stv<VEC>(Vc + r * VT + c, v);
     }
   }
@@ -158,12 +161,10 @@ ml_state_kernel(MlstmArgs a, const int* __restrict__ tiles, float* __restrict__ 
     }
   }
   if (blockIdx.z == 0) {
-    if (tid < LC) gi_s[tid] = tid < L ? expf(gi_s[tid] - b_s[tid] - xl) : 0.f;
-    __syncthreads();
     for (int d = tid; d < D; d += THREADS) {
       float sum = 0.f;
 #pragma unroll 8
-      for (int s = 0; s < LC; ++s) sum = fmaf(gi_s[s], Kt[s * ldk + d], sum);
+      for (int s = 0; s < LC; ++s) sum = fmaf(u_s[s], Kt[s * ldk + d], sum);
       key_sums[((int64_t)blockIdx.x * a.H + h) * D + d] = sum;
     }
   }
@@ -199,7 +200,8 @@ ml_walk_kernel(MlstmArgs a, MlRun* runs, float* states, float* key_sums, const i
   MlRun* run = runs + (int64_t)c0 * a.H + h;
   // The loads of the next AHEAD runs are on their way while these runs' states are stored.
   constexpr int AHEAD = 4;
-  float u[2][AHEAD][VEC], bl[2][AHEAD], xl[2][AHEAD];
+  float u[2][AHEAD][VEC];
+  double bl[2][AHEAD], xl[2][AHEAD];
   auto fetch = [&](int into, int c1) {
 #pragma unroll
     for (int j = 0; j < AHEAD; ++j) {
@@ -220,8 +222,8 @@ ml_walk_kernel(MlstmArgs a, MlRun* runs, float* states, float* key_sums, const i
       for (int j = 0; j < AHEAD; ++j) {
         if (c1 + j < n_runs) {
           stv<VEC>(st + (c1 + j) * step, S);
-          const float m1 = bl[half][j] + fmaxf(m0, xl[half][j]);
-          const float f = expf(bl[half][j] + m0 - m1), g = expf(bl[half][j] + xl[half][j] - m1);
+          const float m1 = (float)(bl[half][j] + fmax((double)m0, xl[half][j]));
+          const float f = expf((float)(bl[half][j] + m0 - m1)), g = expf((float)(bl[half][j] + xl[half][j] - m1));
           if (e == 0) {
             run[(int64_t)(c1 + j) * a.H].m0 = m0;
             run[(int64_t)(c1 + j) * a.H].m1 = m1;
@@ -242,7 +244,8 @@ __global__ void __launch_bounds__(THREADS)
 ml_out_kernel(MlstmArgs a, const int* __restrict__ tiles, const float* __restrict__ states, const float* __restrict__ key_sums,
               const MlRun* __restrict__ runs) {
   extern __shared__ __align__(16) float smem[];
-  __shared__ float bm_s[LC], w_s[LC], c_s[LC], em_s[LC], den_s[LC];
+  __shared__ double top_s[LC], w_s[LC];         // m_t - b_t, gi_t - b_t
+  __shared__ float c_s[LC], em_s[LC], den_s[LC];
   constexpr int lda = LC + 4;
   const int D = a.D, V = a.V, D4 = (D + 3) / 4 * 4, ldq = D4 + 4;
   float* Q = smem;                              // [LC][ldq], times q_scale
@@ -258,11 +261,11 @@ ml_out_kernel(MlstmArgs a, const int* __restrict__ tiles, const float* __restric
   if (L <= 0 || slot < 0) return;
   const MlRun& run = runs[(int64_t)blockIdx.x * a.H + h];
   if (tid < LC) {
-    const float bt = run.b[tid], m0 = run.m0, top = fmaxf(m0, run.x[tid]);       // m_t = b_t + top
-    bm_s[tid] = top;                            // b_t - m_t, negated
-    w_s[tid] = run.gi[tid] - bt;
-    c_s[tid] = expf(m0 - top);
-    em_s[tid] = expf(-(bt + top));
+    const double top = fmax((double)run.m0, run.x[tid]);
+    top_s[tid] = top;
+    w_s[tid] = run.w[tid];
+    c_s[tid] = expf((float)(run.m0 - top));
+    em_s[tid] = expf(-(float)(run.b[tid] + top));
     if (tid == 0 && blockIdx.z == 0 && left <= LC) a.m[(int64_t)slot * a.H + h] = run.m1;
   }
   const float* rows = a.proj + (int64_t)tok0 * a.ld;
@@ -293,7 +296,7 @@ ml_out_kernel(MlstmArgs a, const int* __restrict__ tiles, const float* __restric
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         const int t = ty + 16 * i, s = tx + 16 * j;
-        A[t * lda + s] = s <= t && t < L ? sc[i][j] * expf(w_s[s] - bm_s[t]) : 0.f;
+        A[t * lda + s] = s <= t && t < L ? sc[i][j] * expf((float)(w_s[s] - top_s[t])) : 0.f;
       }
   }
   __syncthreads();                              // K is read, A is written

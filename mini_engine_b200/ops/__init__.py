@@ -1152,7 +1152,7 @@ def polynorm(z: torch.Tensor, coef: torch.Tensor, eps: float, out: torch.Tensor)
 
 # ---- the matrix-memory recurrence ------------------------------------------------------------------
 MLSTM_CHUNK = 64          # tokens per run of the recurrence's prompt kernels (csrc/mlstm_runs.cu)
-MLSTM_RUN = 3 * MLSTM_CHUNK + 4   # float32 values that hold a run's numbers of one head
+MLSTM_RUN = 6 * MLSTM_CHUNK + 4   # float32 values that hold a run's numbers of one head
 mlstm_chunks = True       # portions of prompts by chunks of tokens (False: token by token, always); a switch for comparisons
 
 

@@ -93,3 +93,25 @@ def test_prompts(ops, H, D, V):
 @pytest.mark.parametrize("H, D, V, lens", [(8, 128, 256, [1] * 64), (8, 64, 128, [1] * 3), (4, 72, 130, [1] * 9 + [3, 5, 40]), (2, 300, 1000, [1, 2, 9])])
 def test_single_tokens(ops, H, D, V, lens):
     check(ops, H, D, V, lens, [0 if b % 5 == 1 else 7 for b in range(len(lens))], [(b * 3) % len(lens) if len(lens) % 3 else b for b in range(len(lens))], chunks=False)
+
+
+def test_weights_behind_a_strong_decay(ops):
+    """Fifty tokens whose forget gates stand at the cap take the sums of the gates to some -750; 14 tokens without decay then weigh about the
+    same.  An output is a sum of 14 terms that weigh, of scores of 4 terms, with weights whose exponents lie within 4: at most 14 + 4 + 4 of
+    float32's rounding steps, as many for the sum of the weights, and a few for exponentials and the division."""
+    H, D, V, T = 4, 4, 64, 64
+    g = torch.Generator(DEV).manual_seed(3)
+    rnd = lambda *s: torch.randn(*s, device=DEV, generator=g)
+    offs = {"q": 0, "k": H * D, "v": 2 * H * D, "i": 2 * H * D + H * V, "f": 2 * H * D + H * V + H}
+    proj = rnd(T, offs["f"] + H)
+    proj[:, :2 * H * D] = proj[:, :2 * H * D].abs()
+    proj[:50, offs["f"]:] -= 200
+    proj[50:, offs["f"]:] += 200
+    bias = torch.zeros(H, device=DEV)
+    state = [torch.zeros(s, device=DEV) for s in ((1, H, D, V), (1, H, D), (1, H))]
+    ref = reference(proj, offs, bias, bias, state, [T], [0], [0], H, D, V)[0][50:]
+    size = reference(torch.cat((proj[:, :2 * H * D], proj[:, 2 * H * D:offs["i"]].abs(), proj[:, offs["i"]:]), 1), offs, bias, bias, state, [T], [0], [0],
+                     H, D, V)[0][50:]
+    o = torch.empty(T, H * V, device=DEV)
+    ops.mlstm_scan(proj, offs, bias, bias, CAP, *state, meta_of([T], [T]), torch.zeros(1, dtype=torch.int32, device=DEV), o, H, D, V, D ** -0.5)
+    assert ((o[50:].double() - ref).abs() <= 64 * 2.0 ** -24 * size).all()
