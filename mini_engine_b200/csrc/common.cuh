@@ -68,6 +68,16 @@ __device__ __forceinline__ float block_sum(float x, float* red /* >= 32 floats o
   return total;
 }
 
+// The same by butterflies over the lanes and then over the warps (up to 32): a result stands five additions behind its warps' sums.
+__device__ __forceinline__ float block_sum_tree(float x, float* red /* >= 32 floats of shared memory */) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = (blockDim.x + 31) >> 5;
+  x = warp_sum(x);
+  __syncthreads();
+  if (lane == 0) red[warp] = x;
+  __syncthreads();
+  return warp_sum(lane < nwarps ? red[lane] : 0.f);
+}
+
 // ---- programmatic dependent launch ---------------------------------------------------------------
 // Every kernel is launched so that it may start while its predecessor in the stream is still running
 // (cudaLaunchAttributeProgrammaticStreamSerialization).  A kernel first fetches what no earlier kernel

@@ -191,21 +191,19 @@ hc_norm_vec_kernel(float* __restrict__ x, int64_t stream_stride, int S, const TY
       for (int s = 0; s < NS; ++s)
         if (s < S) v = fmaf(c_in[s], xs[s][c][e], v);
       u[c][e] = v;
-      sum += v;
     }
+    sum += (u[c][0] + u[c][1]) + (u[c][2] + u[c][3]);
   }
   if (normw == nullptr) return;                 // the update alone
-  const float mean = block_sum(sum, red) / (float)W;
+  const float mean = block_sum_tree(sum, red) / (float)W;
   float sq = 0.f;
 #pragma unroll
   for (int c = 0; c < CH; ++c)
-    if (at[c] < W)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const float d = u[c][e] - mean;
-        sq = fmaf(d, d, sq);
-      }
-  const float rstd = 1.0f / sqrtf(block_sum(sq, red) / (float)W + eps);
+    if (at[c] < W) {
+      const float d0 = u[c][0] - mean, d1 = u[c][1] - mean, d2 = u[c][2] - mean, d3 = u[c][3] - mean;
+      sq += fmaf(d0, d0, d1 * d1) + fmaf(d2, d2, d3 * d3);
+    }
+  const float rstd = 1.0f / sqrtf(block_sum_tree(sq, red) / (float)W + eps);
 #pragma unroll
   for (int c = 0; c < CH; ++c) {
     if (at[c] >= W) continue;

@@ -53,14 +53,17 @@ polynorm_vec_kernel(const TZ* __restrict__ z, int64_t ldz, const float* __restri
   }
   float s2 = 0.f, s4 = 0.f, s6 = 0.f;
 #pragma unroll
-  for (int i = 0; i < CH; ++i)
+  for (int i = 0; i < CH; ++i) {
+    float x2[4], x3[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-      const float x2 = v[i][k] * v[i][k];
-      s2 += x2;
-      s4 = fmaf(x2, x2, s4);
-      s6 = fmaf(x2 * v[i][k], x2 * v[i][k], s6);
+      x2[k] = v[i][k] * v[i][k];
+      x3[k] = x2[k] * v[i][k];
     }
+    s2 += (x2[0] + x2[1]) + (x2[2] + x2[3]);
+    s4 += fmaf(x2[0], x2[0], x2[1] * x2[1]) + fmaf(x2[2], x2[2], x2[3] * x2[3]);
+    s6 += fmaf(x3[0], x3[0], x3[1] * x3[1]) + fmaf(x3[2], x3[2], x3[3] * x3[3]);
+  }
   s2 = warp_sum(s2);
   s4 = warp_sum(s4);
   s6 = warp_sum(s6);
@@ -70,12 +73,9 @@ polynorm_vec_kernel(const TZ* __restrict__ z, int64_t ldz, const float* __restri
     red[2][warp] = s6;
   }
   __syncthreads();
-  s2 = s4 = s6 = 0.f;
-  for (int w = 0; w < warps; ++w) {
-    s2 += red[0][w];
-    s4 += red[1][w];
-    s6 += red[2][w];
-  }
+  s2 = warp_sum(lane < warps ? red[0][lane] : 0.f);
+  s4 = warp_sum(lane < warps ? red[1][lane] : 0.f);
+  s6 = warp_sum(lane < warps ? red[2][lane] : 0.f);
   const float r1 = 1.0f / sqrtf(s2 / (float)F + eps), r2 = 1.0f / sqrtf(s4 / (float)F + eps), r3 = 1.0f / sqrtf(s6 / (float)F + eps);
   TO* o = out + (int64_t)blockIdx.x * ldo;
 #pragma unroll

@@ -114,6 +114,30 @@ def test_mlstm_out(ops, H, V, gate, shared):
     near(*outs)
 
 
+# The statistics of a row come from sums of pairs, so that the form's results lie no further from 64 bits than the general form's (thousands of
+# values: the distances themselves vary by some 0.3%).
+@pytest.mark.parametrize("W", [1024, 2048, 4096, 8192, 12288, 16384])
+def test_forms_are_as_close_to_64_bits(ops, W):
+    g = torch.Generator(DEV).manual_seed(W)
+    T, far = 2000, {}
+    x, w = torch.randn(1, T, W, device=DEV, generator=g) * 3 + 1, torch.rand(W, device=DEV, generator=g) + 0.5
+    coef = torch.tensor([0.7, -0.4, 0.9, 0.1], device=DEV)
+    d = x[0].double() - x[0].double().mean(-1, keepdim=True)
+    p, unit = x[0].double(), lambda t: t / torch.sqrt(t.square().mean(-1, keepdim=True) + 1e-5)
+    a, b, c, e = coef.double()
+    refs = {"hc_norm": d / torch.sqrt(d.square().mean(-1, keepdim=True) + 1e-5) * w.double(), "polynorm": a * unit(p) + b * unit(p ** 2) + c * unit(p ** 3) + e}
+    for form in ("vectors", "general"):
+        out = torch.empty(T, W, device=DEV)
+        if W <= 4096:
+            ops.hc_norm(x, norm_weight=w if form == "vectors" else off(w), eps=1e-5, out=out)
+            far["hc_norm", form] = (out.double() - refs["hc_norm"]).norm()
+        ops.polynorm(x[0] if form == "vectors" else off(x[0]), coef, 1e-5, out)
+        far["polynorm", form] = (out.double() - refs["polynorm"]).norm()
+    for name in refs:
+        if (name, "general") in far:
+            assert far[name, "vectors"] <= 1.003 * far[name, "general"]
+
+
 # The sum of a head's squares has one order in all forms: every 32nd value a lane, then a butterfly over the lanes.  Worked out here with numpy
 # (fused multiply-adds through 64 bits), the results are the same to the bit.  Heads of one value to beyond the form in registers.
 @pytest.mark.parametrize("H, V", [(1, 4), (2, 33), (5, 128), (8, 132), (8, 256), (3, 510), (3, 512), (2, 516)])
