@@ -60,6 +60,7 @@ class _StepGraph:
         self.logits: Optional[torch.Tensor] = None
         self.tokens: Optional[torch.Tensor] = None
         self.launches = 0
+        self.buffers: list = []                  # the work buffers' storages at the time of the capture
         self.form: Optional[str] = None          # the decode attention form the capture was tuned to, if it was
 
 
@@ -490,6 +491,7 @@ class ModelRunner:
             gc.enable()
         g.launches = ops.launches - before
         g.graph = graph
+        g.buffers = g.ctx.storages()
 
     def _capture_fastest_form(self, g: _StepGraph, token_ids: torch.Tensor) -> None:
         """Capture a decode step once for every form of the decode attention kernel that takes the shape, replay each a
@@ -522,12 +524,12 @@ class ModelRunner:
                 e1.synchronize()
                 t = e0.elapsed_time(e1)
                 if best is None or t < best[0]:
-                    best = (t, form, g.graph, g.logits, g.tokens, g.launches)
+                    best = (t, form, g.graph, g.logits, g.tokens, g.launches, g.buffers)
                 if t / 4 > self.tune_decode_max_step_ms:
                     break                            # a long step (large layers): the forms differ by a per cent of it at most
         finally:
             ops.decode_form = "auto"
-        _, g.form, g.graph, g.logits, g.tokens, g.launches = best
+        _, g.form, g.graph, g.logits, g.tokens, g.launches, g.buffers = best
 
     def _step_prefill_graph(self, items: Sequence[StepItem], sample: bool) -> Optional[StepResult]:
         """One request's portion of a prompt from a graph; None while the shape has not come twice.

@@ -59,7 +59,7 @@ class StepContext:
         self.device = runner.device
         self.error_flag: torch.Tensor = runner.error_flag
         self._arena: dict[str, torch.Tensor] = {} if arena is None else arena
-        self._views: dict = {}
+        self._views: dict = {}         # name -> (storage, {(shape, dtype): view of it})
         self.frozen = False            # a captured graph's buffers must not be reallocated
         self.on_replace = None         # called with a buffer's name before a larger one takes its place
         self.token_feedback = getattr(runner, "token_feedback", None)   # int32 on the device: a token id ~j in a step means entry j of it
@@ -82,27 +82,41 @@ class StepContext:
         return self._runner()
 
     def buffer(self, name: str, shape, dtype: torch.dtype, zero: bool = False) -> torch.Tensor:
-        """A work buffer by name: the same storage every step, grown when a step needs more.
+        """A work buffer by name: the same storage every step, grown when a step needs more (the smaller storage goes back to the
+        allocator once no tensor of it is left; a captured graph keeps those it recorded).
         ``zero``: the storage is zeroed when it is made (for counters that kernels leave at zero)."""
-        key = (name, tuple(shape), dtype)
-        hit = self._views.get(key)
-        if hit is not None and hit[0] is self._arena.get(name):
-            return hit[1]
+        key = (tuple(shape), dtype)
+        flat = self._arena.get(name)
+        kept = self._views.get(name)
+        if kept is not None:
+            if kept[0] is flat:
+                hit = kept[1].get(key)
+                if hit is not None:
+                    return hit
+            else:
+                del self._views[name]                   # views would keep a storage that was replaced
         n = 1
         for s in shape:
             n *= int(s)
         nbytes = max(n * dtype.itemsize, 16)
-        flat = self._arena.get(name)
         if flat is None or flat.numel() < nbytes:
             if self.frozen:
                 raise RuntimeError(f"work buffer {name!r} would move under a captured graph")
-            if flat is not None and self.on_replace is not None:
-                self.on_replace(name)               # others that recorded the old storage must forget it
+            if flat is not None:
+                if self.on_replace is not None:
+                    self.on_replace(name)           # others that recorded the old storage must forget it
+                if flat.is_cuda:
+                    flat.record_stream(torch.cuda.current_stream())     # launches that still read it may not be on its own stream
+            self._views.pop(name, None)
             flat = (torch.zeros if zero else torch.empty)(nbytes + (-nbytes) % 256, dtype=torch.uint8, device=self.device)
             self._arena[name] = flat
         view = flat[:n * dtype.itemsize].view(dtype).view(*shape)
-        self._views[key] = (flat, view)              # the same tensor object until the storage is replaced
+        self._views.setdefault(name, (flat, {}))[1][key] = view      # the same tensor object until the storage is replaced
         return view
+
+    def storages(self) -> list:
+        """The storages of all work buffers as they are now."""
+        return list(self._arena.values())
 
     def kv_cache(self, cache_slot: int, name: str = "") -> KVView:
         """``name``: which cache, for a layer that asked for several (``KVCacheNeed.name``)."""
