@@ -60,6 +60,7 @@ class StepContext:
         self.error_flag: torch.Tensor = runner.error_flag
         self._arena: dict[str, torch.Tensor] = {} if arena is None else arena
         self._views: dict = {}         # name -> (storage, {(shape, dtype): view of it})
+        self.recorded = arena is not None        # the context of steps that are captured and have one shape
         self.frozen = False            # a captured graph's buffers must not be reallocated
         self.on_replace = None         # called with a buffer's name before a larger one takes its place
         self.token_feedback = getattr(runner, "token_feedback", None)   # int32 on the device: a token id ~j in a step means entry j of it
@@ -113,6 +114,14 @@ class StepContext:
         view = flat[:n * dtype.itemsize].view(dtype).view(*shape)
         self._views.setdefault(name, (flat, {}))[1][key] = view      # the same tensor object until the storage is replaced
         return view
+
+    def most_runs(self, tokens: int) -> int:
+        """Into how many runs of ``tokens`` tokens the requests with several tokens of any step within the runner's limits are cut at most
+        (0 for a captured step: its own shape is all there will be)."""
+        if self.recorded:
+            return 0
+        T = self.runner.max_num_batched_tokens
+        return (T + (tokens - 1) * min(self.runner.max_num_seqs, T // 2)) // tokens
 
     def storages(self) -> list:
         """The storages of all work buffers as they are now."""

@@ -1158,11 +1158,12 @@ mlstm_chunks = True       # portions of prompts by chunks of tokens (False: toke
 
 def mlstm_scan(proj: torch.Tensor, offsets: dict, bias_i: torch.Tensor, bias_f: torch.Tensor, gate_cap: float,
                S: torch.Tensor, n: torch.Tensor, m: torch.Tensor, meta, state_slots: torch.Tensor, o: torch.Tensor,
-               num_heads: int, dim: int, vdim: int, q_scale: float) -> None:
+               num_heads: int, dim: int, vdim: int, q_scale: float, most_runs: int = 0) -> None:
     """Walks every request's tokens of this step through the recurrence from the state in its slot (see csrc/mlstm.cu).
     ``proj`` [T, N] float32 holds q, k, v, i, f at the column ``offsets``; ``o`` [T, heads * vdim] float32.  The
     requests that bring several tokens take MLSTM_CHUNK tokens at a time, all runs of the step side by side (``mlstm_chunks``; their states
-    and numbers lie in the step's workspace), heads of up to 256 keys."""
+    and numbers lie in the step's workspace), heads of up to 256 keys.  ``most_runs``: how many runs a later step may have; the workspace is
+    made for as many at once, so that it does not grow when the memory is given out."""
     T = proj.shape[0]
     _need(proj.dtype == torch.float32 and proj.stride(1) == 1, "mlstm_scan: projections must be float32 rows")
     _need(all(t.dtype == torch.float32 and t.is_contiguous() for t in (S, n, m, o, bias_i, bias_f)), "mlstm_scan: float32 state")
@@ -1174,7 +1175,7 @@ def mlstm_scan(proj: torch.Tensor, offsets: dict, bias_i: torch.Tensor, bias_f: 
     if chunked:
         # an upper bound of the runs that depends on the step's shape only, so that a recorded step keeps its workspace
         multi = meta.num_reqs - meta.num_decodes
-        runs = max(n_tiles, (T - meta.num_decodes) // MLSTM_CHUNK + multi)
+        runs = max(n_tiles, (T - meta.num_decodes) // MLSTM_CHUNK + multi, most_runs)
         states = meta.workspace("mlstm_states", (runs, num_heads, dim, vdim + 1), torch.float32)
         numbers = meta.workspace("mlstm_runs", (runs, num_heads, MLSTM_RUN), torch.float32)
     _call("me_mlstm_scan", proj.data_ptr(), proj.stride(0), offsets["q"], offsets["k"], offsets["v"], offsets["i"], offsets["f"],

@@ -62,7 +62,7 @@ class MLSTM(Mixer):
         o = ctx.buffer("mlstm_o", (T, H * V), torch.float32)
         slot = call.cache_slot
         ops.mlstm_scan(proj, self.offsets, self.p("i.b"), self.p("f.b"), self.gate_cap, ctx.state(slot, "S"), ctx.state(slot, "n"),
-                       ctx.state(slot, "m"), ctx.attn_meta, ctx.state_slots, o, H, D, V, D ** -0.5)
+                       ctx.state(slot, "m"), ctx.attn_meta, ctx.state_slots, o, H, D, V, D ** -0.5, ctx.most_runs(ops.MLSTM_CHUNK))
         gated = ctx.buffer("mlstm_gated", (T, H * V), ctx.act_dtype)
         ops.mlstm_out(o, proj, self.offsets["g"], self.p("norm"), self.norm_eps, gated, H, V)
         return self.o_proj.forward(gated, ctx, "mixer_out")

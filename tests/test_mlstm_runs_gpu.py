@@ -115,3 +115,26 @@ def test_weights_behind_a_strong_decay(ops):
     o = torch.empty(T, H * V, device=DEV)
     ops.mlstm_scan(proj, offs, bias, bias, CAP, *state, meta_of([T], [T]), torch.zeros(1, dtype=torch.int32, device=DEV), o, H, D, V, D ** -0.5)
     assert ((o[50:].double() - ref).abs() <= 64 * 2.0 ** -24 * size).all()
+
+
+def test_the_workspace_is_made_once(ops):
+    """Steps of ever more runs, within an engine's limits, leave the recurrence's workspaces where the first prompt put them."""
+    import logozen_models as zoo
+    from mini_engine_b200 import LLM
+    from mini_engine_b200.cache.manager import CacheHolder
+    from mini_engine_b200.engine.model_runner import StepItem
+    llm = LLM(zoo.folder("P"), dtype="bfloat16", kvcache_block_size=16, num_kvcache_blocks=64, max_num_seqs=4, max_num_batched_tokens=300,
+              max_model_len=400)
+    places = set()
+    for lens in ([2], [70, 3], [200], [65, 65, 65, 65], [258, 2, 2, 2]):
+        items = []
+        for n in lens:
+            h = CacheHolder()
+            assert llm.cache.allocate(h, n)
+            items.append(StepItem(h, [i % 97 for i in range(n)], 0, [n - 1]))
+        llm.model_runner.step(items)
+        for it in items:
+            llm.cache.free(it.holder)
+        arena = llm.model_runner.ctx._arena
+        places.add((arena["mlstm_states"].data_ptr(), arena["mlstm_runs"].data_ptr()))
+    assert len(places) == 1

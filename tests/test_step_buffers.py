@@ -47,3 +47,23 @@ def test_contexts_that_share_an_arena_follow_a_storage_that_another_replaced():
         assert "captured graph" in str(e)
     else:
         raise AssertionError("a frozen context moved a buffer")
+
+
+def test_runs_of_a_step_within_the_limits():
+    runner = Runner()
+    for T, B in ((256, 4), (4096, 64), (100, 512), (16384, 512)):
+        runner.max_num_batched_tokens, runner.max_num_seqs = T, B
+        most = max(sum(-(-n // 64) for n in lens) for lens in _divisions(T, B))
+        assert most <= StepContext(runner).most_runs(64) <= 1.02 * most + 1
+        assert StepContext(runner, {}).most_runs(64) == 0
+
+
+def _divisions(T, B):
+    """Steps of T tokens and up to B requests with two tokens and more that are cut into many runs: all but the last just beyond whole runs."""
+    for n in range(1, min(B, T // 2) + 1):
+        for extra in (2, 65, 129):
+            lens = [extra] * (n - 1)
+            if sum(lens) + 2 <= T:
+                yield lens + [T - sum(lens)]
+        k = (T - 2 * n) // 64                 # two tokens each, then whole runs for as many as there are tokens left
+        yield [2 + 64 * (k // n + (i < k % n)) for i in range(n)]
