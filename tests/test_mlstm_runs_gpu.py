@@ -38,7 +38,7 @@ def make(H, D, V, lens, slots, seed):
     proj = rnd(T, width + 1)[:, :width] if D % 4 else rnd(T, (width + 3) // 4 * 4)
     proj[:, :2 * H * D] = proj[:, :2 * H * D].abs()
     offs = {"q": 0, "k": H * D, "v": 2 * H * D, "i": 2 * H * D + H * V, "f": 2 * H * D + H * V + H}
-    proj[200:300, offs["i"]:offs["i"] + H] += 12                         # gates near the cap: the running maximum rises and stays
+    proj[T // 3:T // 2 + 1, offs["i"]:offs["i"] + H] += 12               # gates near the cap: the running maximum rises and stays
     return proj, offs, rnd(H), rnd(H) + 3, (rnd(slots, H, D, V), rnd(slots, H, D).abs(), rnd(slots, H).abs())
 
 
@@ -89,10 +89,12 @@ def test_prompts(ops, H, D, V):
 
 
 # token by token: more blocks than the device holds at once, so that some start when others have ended; several tokens a request; heads and values
-# beyond the prompt kernels' sizes
+# beyond the prompt kernels' sizes; one request without a slot
 @pytest.mark.parametrize("H, D, V, lens", [(8, 128, 256, [1] * 64), (8, 64, 128, [1] * 3), (4, 72, 130, [1] * 9 + [3, 5, 40]), (2, 300, 1000, [1, 2, 9])])
 def test_single_tokens(ops, H, D, V, lens):
-    check(ops, H, D, V, lens, [0 if b % 5 == 1 else 7 for b in range(len(lens))], [(b * 3) % len(lens) if len(lens) % 3 else b for b in range(len(lens))], chunks=False)
+    slots = [(b * 3) % len(lens) if len(lens) % 3 else b for b in range(len(lens))]
+    slots[1] = -1
+    check(ops, H, D, V, lens, [0 if b % 5 == 2 else 7 for b in range(len(lens))], slots, chunks=False)
 
 
 def test_weights_behind_a_strong_decay(ops):

@@ -35,3 +35,18 @@ def test_parallel_norm(ops, W, n, full):
     for w, b, out in norms:
         ref = unit * w.double() + (b.double() if b is not None else 0.0)
         assert ((out - ref).abs() <= TOL * unit.abs().max() * (w.abs().max() + 1)).all()
+
+
+# which form runs is a matter of the number of rows, which a row's result does not show
+@pytest.mark.parametrize("W", [4, 260, 1028, 2048, 4096])
+@pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
+def test_a_row_among_few_and_among_many(ops, W, dt):
+    g = torch.Generator(DEV).manual_seed(W)
+    x, ya, yb = (torch.randn(700, W, device=DEV, generator=g) for _ in range(3))
+    va, w1, b1, w2 = (torch.randn(W, device=DEV, generator=g) for _ in range(4))
+    res = []
+    for n in (700, 3):
+        s, out1, out2 = x[:n].clone(), torch.empty(n, W, device=DEV, dtype=dt), torch.empty(n, W, device=DEV, dtype=dt)
+        ops.parallel_norm(s, [ya[:n].bfloat16(), yb[:n].bfloat16()], [va], 1e-5, (w1, b1), out1, (w2, None), out2)
+        res.append((s[:3], out1[:3], out2[:3]))
+    assert all(torch.equal(a, b) for a, b in zip(*res))
