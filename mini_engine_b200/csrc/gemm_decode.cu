@@ -34,8 +34,8 @@ __device__ __forceinline__ bf16* dl_ptr(bf16* base, int row, int piece) {
 // EPI 2: residual_out[m][n] += v, sumsq_out, and with ``next_w`` also xw_out[m][n] = residual_out[m][n] * next_w[n].
 // R: weight rows of a strip (16, or 8 with the upper half of the tile idle); XR: rows of X that are held (8 for up to 8 rows, with the
 // upper n8 tile left out).  Shared memory holds no more than these: how many blocks an SM takes decides how much of the weights is
-// in flight (K = 2,048, strips of 16: one block an SM with 16 rows of X, two with 8: 34 MB of
-// weights 18.4 -> 14.4 us with the launch, caches cold; K = 1,024, 17 MB: 14.3 -> 10.3).
+// in flight (K = 2,048, strips of 16: one block an SM with 16 rows of X, two with 8: 34 MB of weights 18.4 -> 14.4 us with the launch,
+// caches cold; K = 1,024, 17 MB: 14.3 -> 10.3).
 template <int EPI, typename TO, int R, int XR>
 __global__ void __launch_bounds__(DL_MAX_WARPS * 32)
 gemm_decode_kernel(const bf16* __restrict__ X, int64_t ldx, const float* __restrict__ sumsq_in, int sumsq_parts, float eps,

@@ -130,8 +130,7 @@ gemm_f32_tile_kernel(const float* __restrict__ A, int64_t lda, const float* __re
   const int m0 = blockIdx.y * ROWS, n0 = blockIdx.x * COLS, stages = (K + TILE_BK - 1) / TILE_BK;
   const int lp = 4 * (tid & 15), lr = tid >> 4;           // a thread brings one piece of every 8th row
   // Inside the matrices a row's place is the thread's first one and a multiple of the same distance; only tiles and stages at an edge
-  // look at each row.  (Each row's address for itself: 154 and 215 us where
-  // q|k|v and gate|up of 613 rows take 150 and 209.)
+  // look at each row.  (Each row's address for itself: 154 and 215 us where q|k|v and gate|up of 613 rows take 150 and 209.)
   const bool inner = m0 + ROWS <= M && n0 + COLS <= N;
   const float* w_first = W + (int64_t)(n0 + lr) * K + lp;
   const float* a_first = A + (int64_t)(m0 + lr) * lda + lp;

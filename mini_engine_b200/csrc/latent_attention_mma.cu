@@ -6,9 +6,9 @@
 // first C columns), for every head.  One block = 64 rows = (64 / gp query tokens) x (gp heads): a key tile is loaded
 // once for gp heads.  Four warps, each a strip of 16 rows; S = Q K^T with Q and K fragments from shared memory by
 // ldmatrix, P rounded to bfloat16 in registers, O += P V with V fragments by transposing ldmatrix from the same tile;
-// key tiles of 64 arrive by cp.async in two buffers, rows padded to a multiple of 64 values and their 16-byte pieces
-// XOR-swizzled.  A block accumulates at most 256 of the C output columns (grid.z takes the others and repeats S).
-// Key tiles start at multiples of 64 from position 0.
+// key tiles of 64 or 32 (lm_tiling) arrive by cp.async in one or two buffers, rows padded to a multiple of 64 values and their
+// 16-byte pieces XOR-swizzled.  A block accumulates at most 256 of the C output columns (grid.z takes the others and repeats S).
+// Key tiles start at multiples of their size from position 0.
 //
 // Portions of prompts: blocks by the step's query-tile list; the softmax's sink and the gate are applied at the end.
 // Single tokens: one block per request, 64 heads and a range of keys; it leaves (max, sum, unnormalised O) in float32,
@@ -31,8 +31,8 @@ __device__ __forceinline__ bf16* tptr(bf16* base, int row, int piece, int ldp) {
 
 // Eight neighbouring threads bring a row's pieces, a thread the rows tid / 8 + 16 i: a page is looked up once a row, all of a thread's
 // before the first copy, and a piece's place takes an addition.  (A thread that went through the tile piece by piece divided three times
-// and waited for a page's number at each: 3 prompts of 300 to 1,300
-// tokens, 16 heads, rows of 256 + 64 values: 366 us, so 260; 3 single tokens behind them 15.4 us, so 11.8.)
+// and waited for a page's number at each: 3 prompts of 300 to 1,300 tokens, 16 heads, rows of 256 + 64 values: 366 us, so 260; 3 single
+// tokens behind them 15.4 us, so 11.8.)
 template <int LM_KEYS>
 __device__ __forceinline__ void load_key_tile(bf16* ks, const bf16* __restrict__ pool, const int* __restrict__ bt,
                                               int page_size, int page_shift, int dk, int pieces, int ldp, int kt, int k_end) {
@@ -132,9 +132,10 @@ latent_attn_mma_kernel(const bf16* __restrict__ q_abs, const bf16* __restrict__ 
 
   // A lane's rows in the tiles, for ldmatrix: of Q 16 warp + .., of K (its columns are K's channels) and of V (the transposed reading).  Rows are
   // whole panels of eight pieces, a lane's row is lane & 7 modulo eight everywhere, so a piece's place in its panel is one of eight numbers
-  // and all else is a distance.  (With places worked out piece by piece 3 single
-  // tokens of 16 heads took 11.8 us, so 9.4.  The prompts' form waits for its products and shared-memory reads, two warps a scheduler:
-  // 235 us either way.)
+  // and all else is a distance.  (With places worked out piece by piece 3 single tokens of 16 heads took 11.8 us, so 9.4.  The prompts' form
+  // waits for its products and shared-memory reads, two warps a scheduler: 235 us either way.  Small latents gained from the loads and the
+  // places together: rows of 128 + 32 values, 3 prompts 162 -> 96 us, 64 single tokens 49 -> 24, 12,000 keys of one 57 -> 27; 64 + 8:
+  // 112 -> 81, 36 -> 22, 47 -> 26; 32 + 16: 76 -> 68, 25 -> 20, 43 -> 25.  Steps over the padding of a row are part of these.)
   const uint32_t row_bytes = ldp * 16, r8 = lane & 7;
   const uint32_t q_at = smem_u32(qs) + (warp * 16 + (mi & 1) * 8 + r8) * row_bytes;
   const uint32_t k_lane = ((mi >> 1) * 8 + r8) * row_bytes, v_lane = ((mi & 1) * 8 + r8) * row_bytes + c0 * 2;

@@ -11,9 +11,8 @@
 // portion starts at position 0) and leaves the new state there; everything is float32, and a token's result does
 // not depend on where the sequence was cut.  One block = one request x one head x MLSTM_VB (16) columns of S; the
 // blocks of a head each keep n and m.  They are stored by a kernel behind (mlstm_norm_kernel), since blocks that start late
-// still read what the slot held.  Portions of prompts run 64 tokens at a time, all
-// runs of a step side by side (mlstm_runs.cu).  A further kernel divides each head's o by its root mean square and
-// applies the weight and the output gate.
+// still read what the slot held.  Portions of prompts run 64 tokens at a time, all runs of a step side by side (mlstm_runs.cu).
+// A further kernel divides each head's o by its root mean square and applies the weight and the output gate.
 #include "mlstm.cuh"
 
 constexpr int MLSTM_VB = 16, MLSTM_DY = 16, MLSTM_THREADS = MLSTM_VB * MLSTM_DY;

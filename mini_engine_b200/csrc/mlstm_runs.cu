@@ -10,10 +10,12 @@
 //   ml_state_kernel   gates, b, x and U of every run: one block = one run x one head x 64 columns
 //   ml_walk_kernel    per request, in order: states[c] <- the state in front of run c
 //   ml_out_kernel     the outputs of a run: scores with their weights, times v, plus q S0, over the denominators
-// What bounds it: float32 multiply-adds on the CUDA cores (D V + D V + 64 (D + V) a token and head) and the states' way through memory
-// (8 D V bytes a run and head there and back).  One kernel that walked a request's runs in order, a block for 16 columns of a head,
-// computed the scores again in each of them and had as many steps behind one another as the longest prompt has runs: 3 prompts of
-// 300 to 1,300 tokens, 8 heads of 128 x 256: 1,064 us, now 59 + 16 + 141.
+// What bounds it: float32 multiply-adds on the CUDA cores (D V for U, D V for q S0, 64 V for the weighted v and 64 D for the scores in each
+// of the V / 64 blocks of a run's outputs: about 3 D V + 64 V a token and head, a quarter of it scores that one block could work out for
+// all) and the states' way through memory (16 D V bytes a run and head: written, read and rewritten by the walk, read for the outputs).
+// One kernel that walked a request's runs in order, a block for 16 columns of a head, worked the scores out in each of them and had as
+// many steps behind one another as the longest prompt has runs: 3 prompts of 300 to 1,300 tokens, 8 heads of 128 x 256: 1,064 us, now
+// 221 in all (under ncu, caches cold, 66 + 24 + 149).
 #include "mlstm.cuh"
 #include "vec4.cuh"
 

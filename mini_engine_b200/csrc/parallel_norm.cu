@@ -139,8 +139,8 @@ parallel_norm_kernel(float* __restrict__ x, const TY* __restrict__ ya, const TY*
 
 // The same sums with a row's values in registers, CH runs of four neighbours a thread (W a multiple of four, at most 1,024 CH): the
 // weights are asked for before the kernel in front has ended and everything of a row together, so that a few rows take one trip to
-// memory.  Bound by that trip and two sums over the block (3 rows of 2,048, two
-// outputs: 6.5 us behind its neighbours in a decode step, so 4.6).
+// memory.  Bound by that trip and two sums over the block (3 rows of 2,048, two outputs: 6.5 us behind its neighbours in a decode
+// step, so 4.6).  The order of the sums is the general form's, so a row's bits do not depend on how many rows there are.
 template <typename TY, typename TO, int CH>
 __global__ void __launch_bounds__(256)
 parallel_norm_regs_kernel(float* __restrict__ x, const TY* __restrict__ ya, const TY* __restrict__ yb, const float* __restrict__ va,
