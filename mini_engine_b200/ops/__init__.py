@@ -32,6 +32,7 @@ _PROTOS = {
     "me_latent_attention": [_P, _P, _I, _P, _P, _I, _P, _P, _P, _I, _I, _P, _P, _P, _I, _I, _I, _I, _I, _F, _I, _P],
     "me_heads_to_rows": [_P, _P, _I, _I, _I, _I, _P],
     "me_latent_attention_mma": [_P, _P, _P, _P, _I, _P, _P, _P, _I, _P, _P, _P, _I, _I, _I, _I, _I, _F, _I, _P],
+    "me_latent_attention_tcgen05": [_P, _P, _P, _P, _I, _P, _P, _P, _I, _P, _P, _P, _I, _I, _I, _I, _I, _F, _I, _P, _P],
     "me_latent_attention_decode": [_P, _P, _P, _P, _I, _P, _P, _I, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _F, _I, _P],
     "me_add_rmsnorm": [_P, _P, _I, _P, _F, _P, _I, _P, _I, _I, _I, _L, _P],
     "me_gemm_skinny": [_P, _L, _P, _P, _I, _L, _P, _I, _I, _I, _I, _P],
@@ -122,6 +123,7 @@ def require_extension() -> ctypes.CDLL:
     lib.me_gemm_skinny_splits.argtypes = [_I]
     lib.me_latent_attention_mma_takes.argtypes = [_I, _I]
     lib.me_latent_attention_mma_heads_per_block.argtypes = [_I]
+    lib.me_latent_attention_tcgen05_heads_per_block.argtypes = [_I, _I, _I, _I]
     _lib = lib
     return lib
 
@@ -1264,6 +1266,7 @@ def gla_chunk_count(meta) -> int:
 # ---- attention through a latent --------------------------------------------------------------------
 LATENT_TILE_Q = 16        # query tokens per block of csrc/latent_attention.cu
 use_latent_mma = True     # bfloat16 latent attention on the tensor cores (csrc/latent_attention_mma.cu); a switch for comparisons
+use_latent_tcgen05 = True # ... and its portions of prompts on tcgen05 (csrc/latent_attention_tcgen05.cu)
 
 
 def latent_decode_plan(num_requests: int, num_heads: int, kv_rank: int, max_context: int) -> tuple[int, int]:
@@ -1292,6 +1295,15 @@ def latent_prep(proj: torch.Tensor, offsets: dict, c_weight: torch.Tensor, eps: 
           q_rot.data_ptr(), _ptr(gate), _dt(pool), T, num_heads, dim, rot_dim, kv_rank, _stream())
 
 
+def latent_tcgen05_heads_per_block(q_abs, q_rot, pool, page_size: int, meta, out, scale: float) -> int:
+    """How many heads share a block of the tcgen05 kernel for portions of prompts; 0 where the mma.sync kernel runs: sizes and pages that
+    the former does not take, rows that a tensor map cannot name, a step without an error word."""
+    if not (use_latent_tcgen05 and scale > 0 and getattr(meta, "error_flag", None) is not None and pool.is_contiguous()
+            and (q_abs.data_ptr() | q_rot.data_ptr() | pool.data_ptr() | out.data_ptr()) % 16 == 0):
+        return 0
+    return (_lib or require_extension()).me_latent_attention_tcgen05_heads_per_block(q_abs.shape[0], q_abs.shape[2], q_rot.shape[2], page_size)
+
+
 def latent_attention(q_abs: torch.Tensor, q_rot: torch.Tensor, pool: torch.Tensor, page_size: int, block_tables: torch.Tensor,
                      meta, sink: Optional[torch.Tensor], gate: Optional[torch.Tensor], out: torch.Tensor, scale: float,
                      window: Optional[int] = None) -> None:
@@ -1305,12 +1317,16 @@ def latent_attention(q_abs: torch.Tensor, q_rot: torch.Tensor, pool: torch.Tenso
     _need(pool.shape[-1] == C + R and pool.dtype == q_abs.dtype, "latent_attention: cache rows")
     lib = _lib or require_extension()
     if q_abs.dtype == torch.bfloat16 and use_latent_mma and lib.me_latent_attention_mma_takes(C, R):
-        # the tensor-core kernels of csrc/latent_attention_mma.cu
-        gp = lib.me_latent_attention_mma_heads_per_block(H)
-        tiles, n_tiles = meta.tile_lists[64 // gp]
+        # the tensor-core kernels of csrc/latent_attention_mma.cu, for portions of prompts of csrc/latent_attention_tcgen05.cu where it takes them
+        tgp = latent_tcgen05_heads_per_block(q_abs, q_rot, pool, page_size, meta, out, scale) if meta.num_decodes < meta.num_reqs else 0
+        tiles, n_tiles = meta.tile_lists[128 // tgp if tgp else 64 // lib.me_latent_attention_mma_heads_per_block(H)]
         common = (q_abs.data_ptr(), q_rot.data_ptr(), pool.data_ptr(), block_tables.data_ptr(), block_tables.stride(0),
                   meta.cu_seqlens.data_ptr(), meta.context_lens.data_ptr())
-        if n_tiles:
+        if n_tiles and tgp:
+            rows = matrix_tensor_map(pool.view(-1, C + R), min(page_size, 64))
+            _call("me_latent_attention_tcgen05", q_abs.data_ptr(), q_rot.data_ptr(), rows.ptr, *common[3:], tiles.data_ptr(), n_tiles, _ptr(sink),
+                  _ptr(gate), out.data_ptr(), T, H, C, R, page_size, float(scale), window, meta.error_flag.data_ptr(), _stream())
+        elif n_tiles:
             _call("me_latent_attention_mma", *common, tiles.data_ptr(), n_tiles, _ptr(sink), _ptr(gate), out.data_ptr(), T, H, C, R,
                   page_size, float(scale), window, _stream())
         D = meta.num_decodes
