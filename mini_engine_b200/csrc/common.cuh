@@ -86,8 +86,9 @@ __device__ __forceinline__ float block_sum_tree(float x, float* red /* >= 32 flo
 // nothing before pdl_wait().  pdl_launch_dependents() lets the successor be scheduled.  In a launch
 // without the attribute both are no-ops.
 // Element-wise activations by number (the keys of ops.ACTIVATIONS): the square of relu, gelu in its tanh form, silu, gelu in its
-// exact form z Phi(z).
-enum { ACT_RELU2 = 0, ACT_GELU_TANH = 1, ACT_SILU = 2, ACT_GELU_ERF = 3 };
+// exact form z Phi(z).  The last is a product's alone: the square of relu of the sum as the product without an epilogue stores it, so
+// that a product and the pass behind it give the same bits as one kernel.
+enum { ACT_RELU2 = 0, ACT_GELU_TANH = 1, ACT_SILU = 2, ACT_GELU_ERF = 3, ACT_RELU2_ROUNDED = 4, ACT_LAST = ACT_RELU2_ROUNDED };
 
 // erf by formula 7.1.26 of Abramowitz and Stegun, Handbook of Mathematical Functions (absolute error up to 1.5e-7), with the fast
 // exponential and reciprocal: for results that are rounded to bfloat16.
@@ -103,8 +104,8 @@ __device__ __forceinline__ float erf_rounded(float x) {
 // TO: the type the result is stored in (bfloat16: short forms with the fast exponential and division).
 template <typename TO = float>
 __device__ __forceinline__ float act_apply(float z, int kind) {
-  if (kind == ACT_RELU2) {
-    const float r = fmaxf(z, 0.f);
+  if (kind == ACT_RELU2 || kind == ACT_RELU2_ROUNDED) {
+    const float r = fmaxf(kind == ACT_RELU2 ? z : to_f<TO>(from_f<TO>(z)), 0.f);
     return r * r;
   }
   if (sizeof(TO) == 2) {
@@ -128,6 +129,7 @@ __device__ __forceinline__ void act_apply_all(float (&g)[N], int kind) {
   if (kind == ACT_RELU2) all(ACT_RELU2);
   else if (kind == ACT_GELU_TANH) all(ACT_GELU_TANH);
   else if (kind == ACT_GELU_ERF) all(ACT_GELU_ERF);
+  else if (kind == ACT_RELU2_ROUNDED) all(ACT_RELU2_ROUNDED);
   else all(ACT_SILU);
 }
 

@@ -272,7 +272,7 @@ ME_API int me_gemm_decode(int epi, const void* X, int64_t ldx, const float* sums
   ME_REQUIRE(X != nullptr && (ldx * 2) % 16 == 0, "me_gemm_decode: X is missing or its rows are not 16-byte aligned");
   ME_REQUIRE(sumsq_in == nullptr || (sumsq_parts > 0 && sumsq_parts <= 192), "me_gemm_decode: sums of squares in %d parts (1..192)",
              sumsq_parts);
-  const int act = epi >= 3 && epi <= 3 + ACT_GELU_ERF ? epi - 3 : -1;
+  const int act = epi >= 3 && epi <= 3 + ACT_LAST ? epi - 3 : -1;
   if (act >= 0) epi = 3;
   ME_REQUIRE(epi == 0 || epi == 1 || (epi == 3 && act >= 0 && y_dtype == ME_BF16) || (epi == 2 && res_out != nullptr && sumsq_out != nullptr), "me_gemm_decode: epilogue %d", epi);
   ME_REQUIRE((next_w == nullptr) == (xw_out == nullptr) && (next_w == nullptr || epi == 2),

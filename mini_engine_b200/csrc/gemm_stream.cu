@@ -342,7 +342,7 @@ ME_API int me_gemm_stream(int epi, const void* map_x, const float* sumsq_in, int
   ME_REQUIRE(map_x != nullptr && map_w != nullptr && err != nullptr && partials != nullptr && flags != nullptr,
              "me_gemm_stream: tensor maps, work buffers and the error word are required");
   ME_REQUIRE(sumsq_in == nullptr || sumsq_parts > 0, "me_gemm_stream: sums of squares in %d parts", sumsq_parts);
-  const int act = epi >= 3 && epi <= 3 + ACT_GELU_ERF ? epi - 3 : -1;
+  const int act = epi >= 3 && epi <= 3 + ACT_LAST ? epi - 3 : -1;
   if (act >= 0) epi = 3;
   ME_REQUIRE(epi == 0 || epi == 1 || (epi == 3 && act >= 0 && y_dtype == ME_BF16) || (epi == 2 && res_out != nullptr && sumsq_out != nullptr), "me_gemm_stream: epilogue %d", epi);
   ME_REQUIRE((next_w == nullptr) == (xw_out == nullptr) && (next_w == nullptr || epi == 2),

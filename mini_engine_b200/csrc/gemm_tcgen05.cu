@@ -861,7 +861,7 @@ ME_API int me_gemm_tcgen05_persistent(const void* map_a, const void* map_w, void
   if (M == 0 || N == 0) return 0;
   ME_REQUIRE(M > 0 && N > 0 && K > 0 && K % 8 == 0, "me_gemm_tcgen05_persistent: bad sizes M=%d N=%d K=%d (K must be a multiple of 8)", M, N, K);
   ME_REQUIRE(map_a != nullptr && map_w != nullptr && err != nullptr, "me_gemm_tcgen05_persistent: tensor maps and the error word are required");
-  ME_REQUIRE(epi == 0 || ((epi == 1 || (epi >= 2 && epi <= 2 + ACT_GELU_ERF)) && c_dtype == ME_BF16), "me_gemm_tcgen05_persistent: epilogue %d", epi);
+  ME_REQUIRE(epi == 0 || ((epi == 1 || (epi >= 2 && epi <= 2 + ACT_LAST)) && c_dtype == ME_BF16), "me_gemm_tcgen05_persistent: epilogue %d", epi);
   ME_REQUIRE(bn == 128 || bn == 256, "me_gemm_tcgen05_persistent: tile width %d is not 128 or 256", bn);
   GluParams glu;
   glu.limit = glu_limit, glu.alpha = glu_alpha, glu.shift = glu_shift;
@@ -919,7 +919,7 @@ ME_API int me_gemm_tcgen05(const void* map_a, const void* map_w, void* C, int c_
   if (M == 0 || N == 0) return 0;
   ME_REQUIRE(M > 0 && N > 0 && K > 0 && K % 8 == 0, "me_gemm_tcgen05: bad sizes M=%d N=%d K=%d (K must be a multiple of 8)", M, N, K);
   ME_REQUIRE(map_a != nullptr && map_w != nullptr && err != nullptr, "me_gemm_tcgen05: tensor maps and the error word are required");
-  ME_REQUIRE(epi == 0 || ((epi == 1 || (epi >= 2 && epi <= 2 + ACT_GELU_ERF)) && c_dtype == ME_BF16), "me_gemm_tcgen05: epilogue %d", epi);
+  ME_REQUIRE(epi == 0 || ((epi == 1 || (epi >= 2 && epi <= 2 + ACT_LAST)) && c_dtype == ME_BF16), "me_gemm_tcgen05: epilogue %d", epi);
   ME_REQUIRE((M + TG_BM - 1) / TG_BM <= 65535, "me_gemm_tcgen05: M=%d is too large", M);
   ME_REQUIRE(splits >= 1 && splits <= 64 && (splits == 1 || (epi == 0 && c_dtype == ME_F32)),
              "me_gemm_tcgen05: %d splits (they need float32 results and no epilogue)", splits);

@@ -49,7 +49,7 @@ def gevulorn_plan(cfg: GevulornConfig) -> ModelPlan:
             mixer = PartSpec("masked_sink_attention", args)
         mlp, ffn = layer["mlp"], None
         if mlp is not None and mlp["kind"] == "dense":
-            ffn = PartSpec("activation_mlp", {"hidden_size": W, "intermediate_size": mlp["ff"], "activation": "relu_squared", "in_product": True})
+            ffn = PartSpec("activation_mlp", {"hidden_size": W, "intermediate_size": mlp["ff"], "activation": "relu_squared", "in_product": "rounded"})
         elif mlp is not None:
             silu_gated = {"limit": None, "alpha": 1.0, "shift": 0.0}
             ffn = PartSpec("routed_experts", {

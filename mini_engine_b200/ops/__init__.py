@@ -465,9 +465,9 @@ def decode_linear(weight: torch.Tensor, x: torch.Tensor, *, out: Optional[torch.
     "residual": residual_out += x W^T; ``sumsq_out`` [decode_linear_sumsq_parts(N), M] gets the new residual's sums
     of squares per strip of columns, and with ``next_norm`` = (weight float32 [N], xw bfloat16 [M, N]) xw gets the new
     residual times that weight).  ``fetch_ahead``: a tensor that a later kernel reads (the next product's weight);
-    this kernel asks it into L2.  ``epilogue`` may also be a key of ``ACTIVATIONS``: that function of the results.  ``glu`` = (limit, alpha, shift) with "silu_mul": the gated epilogue in its general form,
+    this kernel asks it into L2.  ``epilogue`` may also be a key of ``PRODUCT_ACTIVATIONS``: that function of the results.  ``glu`` = (limit, alpha, shift) with "silu_mul": the gated epilogue in its general form,
     g sigmoid(alpha g) (u + shift) with g = min(gate, limit), u = clamp(up, -limit, limit) when limit > 0."""
-    epi = 3 + ACTIVATIONS[epilogue] if epilogue in ACTIVATIONS else {"none": 0, "silu_mul": 1, "residual": 2}[epilogue]
+    epi = 3 + PRODUCT_ACTIVATIONS[epilogue] if epilogue in PRODUCT_ACTIVATIONS else {"none": 0, "silu_mul": 1, "residual": 2}[epilogue]
     _need(glu is None or epi == 1, "decode_linear: the gate's parameters go with the gated epilogue")
     glu_params = tuple(float(v) for v in (glu or (0.0, 1.0, 0.0)))
     M, K = x.shape
@@ -603,12 +603,12 @@ def linear_tcgen05(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, epi
 
     ``glu`` = (limit, alpha, shift) with the "silu_mul" epilogue: the gated epilogue in its general form,
     g sigmoid(alpha g) (u + shift) with g = min(gate, limit), u = clamp(up, -limit, limit) when limit > 0.  ``epilogue`` may also
-    be a key of ``ACTIVATIONS``: that function of the results (bfloat16).
+    be a key of ``PRODUCT_ACTIVATIONS``: that function of the results (bfloat16).
 
     With ``splits`` > 1 ``out`` is float32 [tcgen05_splits(K, splits), M, N]: partial results over parts of K.
     ``share``: the form that cuts the stages of all tiles into one equal range an SM (``tile_n`` 128 or 256)."""
     M, K = x.shape
-    act = 2 + ACTIVATIONS[epilogue] if epilogue in ACTIVATIONS else 0       # (as for no epilogue, but for the call itself)
+    act = 2 + PRODUCT_ACTIVATIONS[epilogue] if epilogue in PRODUCT_ACTIVATIONS else 0       # (as for no epilogue, but for the call itself)
     epi = 0 if act else {"none": 0, "silu_mul": 1}[epilogue]
     _need(not act or (splits == 1 and out.dtype == torch.bfloat16), "linear_tcgen05: an activation goes with whole sums and bfloat16 results")
     _need(glu is None or epi == 1, "linear_tcgen05: the gate's parameters go with the gated epilogue")
@@ -691,9 +691,15 @@ def tcgen05_split_plan(M: int, N: int, K: int) -> tuple[int, int]:
 
 
 def linear_activation_takes(x: torch.Tensor, weight: torch.Tensor, out: Optional[torch.Tensor], err: Optional[torch.Tensor]) -> bool:
-    """Whether ``linear`` takes a key of ``ACTIVATIONS`` as epilogue for these operands: the tcgen05 kernels do."""
+    """Whether ``linear`` takes a key of ``PRODUCT_ACTIVATIONS`` as epilogue for these operands: the tcgen05 kernels do."""
     return (err is not None and use_tcgen05_gemm and skinny_splits(x.shape[0], x.shape[1], x, weight) == 0 and tcgen05_takes(x, weight)
             and (out is None or out.dtype == torch.bfloat16))
+
+
+def linear_shares_work(x: torch.Tensor, weight: torch.Tensor) -> bool:
+    """Whether ``linear`` without an epilogue runs these operands on the work-sharing form of the tcgen05 product, which adds a tile's sums
+    in parts: with an activation for epilogue they run another form, and the sums' last bits differ."""
+    return tcgen05_share == "auto" and tcgen05_share_pays(x.shape[0], weight.shape[0], x.shape[1], 0)
 
 
 def linear(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, epilogue: str = "none",
@@ -722,7 +728,7 @@ def linear(x: torch.Tensor, weight: torch.Tensor, out: torch.Tensor, epilogue: s
     M, K = x.shape
     _need(weight.dim() == 2 and weight.shape[1] == K and weight.is_contiguous(), "linear: weight shape")
     _need(x.stride(1) == 1 and out.stride(1) == 1, "linear: rows must be contiguous")
-    if epilogue in ACTIVATIONS:
+    if epilogue in PRODUCT_ACTIVATIONS:
         _need(linear_activation_takes(x, weight, out, err), "linear: no kernel of this shape applies an activation to its results")
         linear_tcgen05(x, weight, out, epilogue, err)
         _remember(key, sig, before)
@@ -1574,6 +1580,9 @@ def gated_group_norm(y: torch.Tensor, z: torch.Tensor, weight: Optional[torch.Te
 
 
 ACTIVATIONS = {"relu_squared": 0, "gelu_tanh": 1, "silu": 2, "gelu": 3}     # "gelu": the exact form, z Phi(z)
+# What a product can apply to its float32 sums: the same, and the square of relu of the sums as the product alone would store them (the
+# bits of that product and ``activation`` behind it).
+PRODUCT_ACTIVATIONS = dict(ACTIVATIONS, relu_squared_rounded=4)
 
 
 def activation(x: torch.Tensor, out: torch.Tensor, kind: str) -> None:

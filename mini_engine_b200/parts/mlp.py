@@ -44,14 +44,19 @@ class SwiGLU(FeedForward):
 class ActivationMLP(FeedForward):
     """``down(act(up(x)))`` with an element-wise activation (a key of ``ops.ACTIVATIONS``; "relu_squared" is max(z, 0)^2).
     ``in_product``: where a kernel of the first product can, it applies the activation to its float32 sums itself; else (and by
-    default) the activation is a pass of its own over the product's results in the working dtype."""
+    default) the activation is a pass of its own over the product's results in the working dtype.  "rounded" (the square of relu): the
+    kernel rounds its sums to the working dtype first, as the pass finds them, so a token's bits are the same either way, however many
+    tokens share its step (a step of 17 to 127 tokens may run a product without the epilogue)."""
     capturable = True
 
     def __init__(self, hidden_size: int, intermediate_size: int, activation: str = "relu_squared", up: str = "up", down: str = "down",
-                 in_product: bool = False):
+                 in_product: bool | str = False):
         super().__init__()
         from .. import ops
-        self.in_product = in_product
+        if in_product == "rounded" and activation != "relu_squared":
+            raise ValueError(f"no product rounds its sums in front of {activation!r}")
+        # the product's epilogue, where its kernel has one
+        self.epilogue = None if not in_product else (activation + "_rounded" if in_product == "rounded" else activation)
         if activation not in ops.ACTIVATIONS:
             raise ValueError(f"unknown activation {activation!r}; known: {sorted(ops.ACTIVATIONS)}")
         self.hidden_size, self.intermediate_size, self.activation = hidden_size, intermediate_size, activation
@@ -66,8 +71,8 @@ class ActivationMLP(FeedForward):
 
     def forward(self, x, ctx, out_name: str = "ffn_out"):
         from .. import ops
-        fused = self.in_product and self.up.fuses(x, ctx, self.activation)
-        z = self.up.forward(x, ctx, out_name + "_up", epilogue=self.activation if fused else "none", fetch_ahead=self.down.weight)
+        fused = self.epilogue is not None and self.up.fuses(x, ctx, self.epilogue)
+        z = self.up.forward(x, ctx, out_name + "_up", epilogue=self.epilogue if fused else "none", fetch_ahead=self.down.weight)
         if not fused:
             act = ctx.buffer(out_name + "_act", tuple(z.shape), ctx.act_dtype)
             ops.activation(z, act, self.activation)

@@ -385,3 +385,30 @@ def test_squared_relu_and_the_cap(dtype):
     ops.soft_cap(zd, 15.0)
     assert torch.allclose(zd.cpu().double(), plain.soft_cap(z.double(), 15.0), atol=2e-5)
     assert zd.abs().max() <= 15.0
+
+
+@pytest.mark.parametrize("W, F", [(256, 520), (52, 70), (2048, 8192), (6144, 1032), (4096, 6144)])
+@pytest.mark.parametrize("T", [1, 16, 17, 47, 48, 127, 128, 300, 1024, 2787])
+def test_squared_relu_in_every_kernel_of_its_product(T, W, F):
+    """The product's epilogue gives the bits of the product with the pass behind it, so a token's do not depend on how many share its step.
+    Against 64 bits: the sum, its square and the result are rounded to bfloat16, 2^-9 each, the sum's twice over as it is squared, which is
+    below 2^-7 of the terms' magnitudes; the float32 sums of up to 8,192 terms take up to 2^-11 more."""
+    from mini_engine_b200.parts import ActivationMLP
+    ops = _ops()
+    up = (torch.randn(F, W, generator=g(1)) * (2.0 / W ** 0.5)).bfloat16().to(DEV)
+    down = (torch.randn(W, F, generator=g(2)) / F ** 0.5).bfloat16().to(DEV)
+    x = torch.randn(T, W, generator=g(3)).bfloat16().to(DEV)
+    ctx = SimpleNamespace(act_dtype=torch.bfloat16, error_flag=torch.zeros(4, dtype=torch.int32, device=DEV),
+                          buffer=lambda name, shape, dtype, zero=False: torch.zeros(shape, dtype=dtype, device=DEV))
+    got = {}
+    for in_product in ("rounded", False):
+        mlp = ActivationMLP(W, F, "relu_squared", in_product=in_product)
+        mlp.up.params["up"], mlp.down.params["down"] = up, down
+        if in_product:
+            in_kernel = W % 8 == 0 and (T <= 16 or T >= (48 if W * F <= 8 << 20 else 128)) and not ops.linear_shares_work(x, up)
+            assert mlp.up.fuses(x, ctx, mlp.epilogue) == in_kernel
+        got[in_product] = mlp.forward(x, ctx)
+    assert not ctx.error_flag.any() and torch.equal(got["rounded"], got[False])
+    act = torch.relu(x.double() @ up.double().t()) ** 2
+    ref, terms = act @ down.double().t(), act @ down.double().abs().t()
+    assert bool(((got["rounded"].double() - ref).abs() <= (2.0 ** -7 + 2.0 ** -11) * terms + 1e-6).all())
