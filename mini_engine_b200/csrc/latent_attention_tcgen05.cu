@@ -42,7 +42,7 @@ latent_attn_tcgen05_kernel(const bf16* __restrict__ q_abs, const bf16* __restric
                            const float* __restrict__ gate, bf16* __restrict__ out, int T_total, int H, int C, int R, int page_size, int box_rows,
                            float scale_log2, int window, int gp, int ring, uint32_t tmem_cols, int* __restrict__ err) {
   extern __shared__ unsigned char lt_smem_raw[];
-  __shared__ __align__(8) unsigned long long q_bar, k_full[LT_RING], k_empty[LT_RING], s_ready[2], p_ready, o_ready;
+  __shared__ __align__(8) unsigned long long q_bar, k_full[LT_RING], k_empty[LT_RING], s_ready[2], p_ready[2], o_ready[2];
   __shared__ uint32_t tmem_slot;
   unsigned char* smem = lt_smem_raw + ((1024u - (tma::smem_addr(lt_smem_raw) & 1023u)) & 1023u);
   const int dk = C + R, blocks = (dk + 63) / 64, key_bytes = blocks * LT_KBLOCK;
@@ -68,10 +68,19 @@ latent_attn_tcgen05_kernel(const bf16* __restrict__ q_abs, const bf16* __restric
       tma::mbar_init(&k_full[s], 1);
       tma::mbar_init(&k_empty[s], 1);
     }
-    tma::mbar_init(&s_ready[0], 1);
-    tma::mbar_init(&s_ready[1], 1);
-    tma::mbar_init(&p_ready, 4);                          // one arrival per softmax warp
-    tma::mbar_init(&o_ready, 1);
+    // Two barriers a kind, taken by the tile's parity.  A barrier counts arrivals, whoever makes them, and a wait names its phase by parity, so
+    // between a tile and the next but one on the same barrier all must have passed:
+    //   p_ready: a warp arrives for tile it + 2 behind S(it + 2), whose product is issued after the wait for P(it), all four arrivals.  So no
+    //     warp arrives twice in a phase, and the issuing warp cannot miss one.  (On one barrier a warp that need not rescale O arrived for
+    //     it + 1 in the place of one that was still rescaling for it.)
+    //   s_ready: S(it + 2) is asked for after P(it), so every warp has passed its wait for S(it).
+    //   o_ready: a wait for P V (it) stands behind S(it + 1), issued after P V (it - 1); the commit behind S covers all products before it, so
+    //     P V (it - 2), the phase before, is over.  P V (it + 2) needs this warp's P(it + 2), so the phase is not passed over either.
+    for (int i = 0; i < 2; ++i) {
+      tma::mbar_init(&s_ready[i], 1);
+      tma::mbar_init(&p_ready[i], 4);                     // one arrival per softmax warp
+      tma::mbar_init(&o_ready[i], 1);
+    }
     tma::mbar_fence_init();
     tma::prefetch_map(&pool_map);
   }
@@ -133,7 +142,7 @@ latent_attn_tcgen05_kernel(const bf16* __restrict__ q_abs, const bf16* __restric
         ok = issue_qk(it + 1);
         if (!ok) break;
       }
-      ok = tc5::mbar_wait_warp(&p_ready, it & 1);         // P(it) is in tensor memory, O is rescaled if it had to be
+      ok = tc5::mbar_wait_warp(&p_ready[it & 1], (it >> 1) & 1);         // P(it) is in tensor memory, O is rescaled if it had to be
       if (!ok) break;
       tc5::fence_after_sync();
       // A = P, 8 columns of tensor memory for 16 keys; B = V: 16 keys are 2048 bytes further in every 64-column block.
@@ -141,7 +150,7 @@ latent_attn_tcgen05_kernel(const bf16* __restrict__ q_abs, const bf16* __restric
       for (int k = 0; k < LT_KEYS / 16; ++k)
         tc5::mma_f16_a_in_tmem_elect(tmem_o, tmem_s + (it & 1) * LT_KEYS + k * 8, v_desc, (s * key_bytes + k * 2048) >> 4, idesc_o,
                                      it > 0 || k > 0);
-      tc5::commit_elect(&o_ready);
+      tc5::commit_elect(&o_ready[it & 1]);
       tc5::commit_elect(&k_empty[s]);
     }
   } else {
@@ -174,7 +183,6 @@ latent_attn_tcgen05_kernel(const bf16* __restrict__ q_abs, const bf16* __restric
     for (int it = 0; it < n_tiles && ok; ++it) {
       const int kt = lo + it * LT_KEYS;
       const uint32_t t_s = tmem_s + (it & 1) * LT_KEYS + t_row;
-      // S(it - 2), the phase before on its barrier, was waited for two tiles ago.
       ok = tc5::mbar_wait_warp(&s_ready[it & 1], (it >> 1) & 1);
       if (!ok) break;
       tc5::fence_after_sync();
@@ -201,8 +209,7 @@ latent_attn_tcgen05_kernel(const bf16* __restrict__ q_abs, const bf16* __restric
         l1 *= alpha;
       }
       if (it > 0 && __any_sync(0xffffffffu, alpha != 1.f)) {
-        // After P V (it - 1).  P V (it - 2), the phase before, is over: Q K^T (it) was issued after it, and S(it) has been waited for.
-        ok = tc5::mbar_wait_warp(&o_ready, (it - 1) & 1);
+        ok = tc5::mbar_wait_warp(&o_ready[(it - 1) & 1], ((it - 1) >> 1) & 1);          // after P V (it - 1)
         if (!ok) break;
         tc5::fence_after_sync();
         for (int c0 = 0; c0 < C; c0 += 32) {               // (the row of S is held meanwhile)
@@ -247,11 +254,10 @@ latent_attn_tcgen05_kernel(const bf16* __restrict__ q_abs, const bf16* __restric
       lt_fence_async_smem();                               // the zeroed rows of V were written by ordinary stores
       tc5::fence_before_sync();
       __syncwarp();
-      if (lane == 0) lt_arrive(&p_ready);
+      if (lane == 0) lt_arrive(&p_ready[it & 1]);
     }
-    // P V (n - 2) first, which nothing so far has waited for: a wait names its phase by parity.
-    if (ok && n_tiles > 1) ok = tc5::mbar_wait_warp(&o_ready, (n_tiles - 2) & 1);
-    if (ok) ok = tc5::mbar_wait_warp(&o_ready, (n_tiles - 1) & 1);
+    // The last P V, and with it all before.  (P V (n - 3), the phase before on that barrier, is over: S(n - 1) was issued after it.)
+    if (ok) ok = tc5::mbar_wait_warp(&o_ready[(n_tiles - 1) & 1], ((n_tiles - 1) >> 1) & 1);
     if (ok) {
       tc5::fence_after_sync();
       float l = l0 + l1;

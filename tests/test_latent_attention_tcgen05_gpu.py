@@ -78,3 +78,53 @@ def test_infinite_scores_and_rows_beside_them():
             ref = _plain_rows_attention(qa[t], qr[t], r, C, 0.2, sink, L - 3 + t)
             assert got[t].isnan().equal(ref.isnan()) and bool(ref[1].isnan().all()) == (key <= L - 3 + t)
             assert torch.allclose(got[t, [0, 2, 3]], ref[[0, 2, 3]], atol=2e-2, rtol=2e-2)
+
+
+@pytest.mark.parametrize("apart", [True, False])
+@pytest.mark.parametrize("C, R, page", [(64, 8, 16), (128, 32, 16), (256, 64, 64)])
+def test_warps_that_rescale_at_every_tile_beside_warps_that_never_do(C, R, page, apart):
+    """Long contexts, two blocks an SM where the sizes allow it.  With 16 heads a warp holds two tokens of a block's eight: those of one warp
+    score higher from tile to tile and the others lower (``apart``), or the other way round, so warps drift apart as far as the barriers let
+    them; the last block has one token, and three warps without any.  Repeated launches agree bit for bit.  Weights, their sum and the result
+    are rounded to bfloat16, 2^-9 each: below 2^-7 of the terms' magnitudes."""
+    H, scale, lens, contexts = 16, 0.25, [1160, 1201], [3000, 4001]
+    gen, ops = g(C + R), _ops()
+    pages = [-(-n // page) for n in contexts]
+    perm = torch.randperm(sum(pages), generator=gen).int()
+    table = torch.zeros(2, max(pages), dtype=torch.int32)
+    pool = torch.full((sum(pages) * page, C + R), float("nan"), dtype=torch.bfloat16)
+    rows = []
+    for b, n in enumerate(contexts):
+        table[b, :pages[b]] = perm[sum(pages[:b]):sum(pages[:b + 1])]
+        rows.append((torch.randn(n, C + R, generator=gen) * 0.5).bfloat16())
+        rows[b][:, 0] = (torch.arange(n) // 64).float() / 8         # (exact in bfloat16)
+        places = (table[b, :pages[b], None].long() * page + torch.arange(page)).flatten()[:n]
+        pool[places] = rows[b]
+    T = sum(lens)
+    qa, qr = (torch.randn(T, H, C, generator=gen) * 0.02).bfloat16(), (torch.randn(T, H, R, generator=gen) * 0.02).bfloat16()
+    local = torch.cat([torch.arange(n) for n in lens])
+    qa[:, :, 0] = torch.where(((local // 2) % 4 == 2) == apart, 10.0, -10.0)[:, None].bfloat16()     # 0.3 a tile, against noise of 0.05
+    sink = torch.randn(H, generator=gen).to(DEV)
+    meta = _meta(lens, contexts)
+    meta.error_flag = torch.zeros(4, dtype=torch.int32, device=DEV)
+    q, qr, pool, table = qa.transpose(0, 1).contiguous().to(DEV), qr.to(DEV), pool.to(DEV), table.to(DEV)
+    first, out = None, torch.empty(H, T, C, dtype=torch.bfloat16, device=DEV)
+    assert ops.latent_tcgen05_heads_per_block(q, qr, pool, page, meta, out, scale) == 16
+    for _ in range(20):
+        out.fill_(float("nan"))
+        ops.latent_attention(q, qr, pool, page, table, meta, sink, None, out, scale)
+        first = out.clone() if first is None else first
+        assert torch.equal(out, first) and not meta.error_flag.any()
+    t0 = 0
+    for b, n in enumerate(contexts):
+        keys = rows[b].to(DEV).double()
+        seen = torch.arange(n, device=DEV)[None] <= torch.arange(n - lens[b], n, device=DEV)[:, None]
+        for h in range(H):
+            s = torch.cat([q[h, t0:t0 + lens[b]], qr[t0:t0 + lens[b], h]], 1).double() @ keys.t() * scale
+            s = torch.where(seen, s, -torch.inf)
+            m = torch.maximum(s.amax(1, keepdim=True), sink[h].double())
+            p = torch.exp(s - m)
+            p = p / (p.sum(1, keepdim=True) + torch.exp(sink[h].double() - m))
+            err = (first[h, t0:t0 + lens[b]].double() - p @ keys[:, :C]).abs()
+            assert bool((err <= 2.0 ** -7 * (p @ keys[:, :C].abs()) + 1e-6).all()), f"request {b}, head {h}"
+        t0 += lens[b]
