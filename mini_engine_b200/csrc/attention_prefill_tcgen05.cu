@@ -404,7 +404,7 @@ attn_prefill_tcgen05_two_groups_kernel(const __grid_constant__ CUtensorMap q_map
   constexpr int HALF_BYTES = 128 * 128, KB_BYTES = KEYS * 128;
   constexpr uint32_t TMEM_COLS = 512;
   extern __shared__ unsigned char ta_smem_raw[];
-  __shared__ __align__(8) unsigned long long q_bar, k_full[RING], k_empty[RING], v_full[RING], v_empty[RING], s_ready[3], p_ready[2],
+  __shared__ __align__(8) unsigned long long q_bar, k_full[RING], k_empty[RING], v_full[RING], v_empty[RING], s_ready[3], p_ready[3],
       o_ready[2];
   __shared__ uint32_t tmem_slot;
   __shared__ float ref_m[2][TA_ROWS];                   // reference(t) of every row, for t even and odd
@@ -455,11 +455,12 @@ attn_prefill_tcgen05_two_groups_kernel(const __grid_constant__ CUtensorMap q_map
       tma::mbar_init(&v_full[s], 1);
       tma::mbar_init(&v_empty[s], 1);
       tma::mbar_init(&s_ready[s], 1);
+      // One arrival per warp of the tile's group; a barrier per S buffer.  The next arrivals on it, for tile it + 3, stand behind S(it + 3),
+      // whose product is issued after the wait for P(it): the issuing warp cannot miss a phase.  (On a barrier per group it could: P(it + 2)
+      // stands behind S(it + 2) only, whose product is issued before that wait.)
+      tma::mbar_init(&p_ready[s], 4);
     }
-    for (int s = 0; s < 2; ++s) {
-      tma::mbar_init(&p_ready[s], 4);                     // one arrival per warp of the group
-      tma::mbar_init(&o_ready[s], 1);
-    }
+    for (int s = 0; s < 2; ++s) tma::mbar_init(&o_ready[s], 1);
     tma::mbar_fence_init();
     tma::prefetch_map(&q_map);
     tma::prefetch_map(&kv_map);
@@ -552,12 +553,12 @@ attn_prefill_tcgen05_two_groups_kernel(const __grid_constant__ CUtensorMap q_map
     if (ok) ok = issue_qk(0);
     if (ok && n_tiles > 1) ok = issue_qk(1);
     for (int it = 0; it < n_tiles && ok; ++it) {
-      const int s = it % RING, g = it & 1;
+      const int s = it % RING;
       if (it + 2 < n_tiles) {                              // two tiles ahead: one for each softmax group
         ok = issue_qk(it + 2);
         if (!ok) break;
       }
-      ok = tc5::mbar_wait_warp(&p_ready[g], (it >> 1) & 1);  // P(it) is in tensor memory, O is rescaled if it had to be
+      ok = tc5::mbar_wait_warp(&p_ready[s], (it / RING) & 1);  // P(it) is in tensor memory, O is rescaled if it had to be
       if (ok) ok = tc5::mbar_wait_warp(&v_full[s], (it / RING) & 1);
       if (!ok) break;
       tc5::fence_after_sync();
@@ -566,7 +567,7 @@ attn_prefill_tcgen05_two_groups_kernel(const __grid_constant__ CUtensorMap q_map
 #pragma unroll
       for (int k = 0; k < KEYS / 16; ++k)
         tc5::mma_f16_a_in_tmem_elect(tmem_o, tmem_s + s * KEYS + k * 8, v_desc, (s * KV_BYTES + k * 2048) >> 4, idesc_o, it > 0 || k > 0);
-      tc5::commit_elect(&o_ready[g]);                      // P V (it) and everything before it are done
+      tc5::commit_elect(&o_ready[it & 1]);                    // P V (it) and everything before it are done
       tc5::commit_elect(&v_empty[s]);
     }
   } else {
@@ -737,7 +738,7 @@ attn_prefill_tcgen05_two_groups_kernel(const __grid_constant__ CUtensorMap q_map
         tc5::fence_before_sync();
       }
       __syncwarp();
-      if (ok && lane == 0) mbar_arrive(&p_ready[g]);
+      if (ok && lane == 0) mbar_arrive(&p_ready[it % 3]);
     }
     // The group that did not take the last tile takes the last reference off its barrier.
     if (g == (n_tiles & 1)) asm volatile("bar.sync %0, 256;\n" ::"r"(2 + ((n_tiles - 1) & 1)) : "memory");

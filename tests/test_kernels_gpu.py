@@ -598,6 +598,30 @@ def test_attention_tensor_core_prefill(ops, nh, nkv, hd, page, window):
     assert ops.prefill_tcgen05_heads_per_block(16, 8, 128, 16) == 2 and ops.prefill_tcgen05_heads_per_block(16, 8, 128, 24) == 0
 
 
+@pytest.mark.parametrize("hd", [64, 128])
+@pytest.mark.parametrize("apart", [True, False])
+def test_tcgen05_prefill_with_warps_that_drift_apart(ops, hd, apart):
+    """Rows of one warp whose scores rise from one 64 keys to the next by more than 2^8, so that it rescales its outputs at every key tile, beside
+    warps whose scores fall and that never do (``apart``), or the other way round: repeated launches agree bit for bit.  A block holds two
+    heads of 64 tokens; the rows are those of its third warp."""
+    nh, nkv, ctx, ql = 16, 8, [3000, 2111], [700, 641]
+    b = Batch(ctx, ql, nh, nkv, hd, 16, torch.bfloat16, seed=hd)
+    for r, L in enumerate(ctx):
+        j = torch.arange(L, device=DEV)
+        b.pool[b.bt[r, j // 16].long(), 0, :, j % 16, 0] = (j // 64).to(torch.bfloat16)[:, None]          # (exact)
+    b.pool[:, 1] *= 0.25                                  # values below 2: a result and its reference may round a bfloat16 step of 2^-7 apart
+    q = b.qkv.view(-1, nh + 2 * nkv, hd)[:, :nh]
+    q *= 0.05
+    local = torch.cat([torch.arange(n, device=DEV) for n in ql])
+    own = (local % 64 < 32)[:, None] & (torch.arange(nh, device=DEV) % 2 == 1)[None]
+    q[:, :, 0] = torch.where(own == apart, 6.0, -6.0).to(torch.bfloat16) * hd ** 0.5
+    for which in ("tcgen05_128",):
+        first, ref = run_attention(ops, b, torch.bfloat16, None, which)
+        close(first, ref, torch.bfloat16)
+        for _ in range(10):
+            assert torch.equal(run_attention(ops, b, torch.bfloat16, None, which)[0], first)
+
+
 @pytest.mark.parametrize("kind", ["cuda_cores", "tensor_cores", "tensor_cores_tma"])
 @pytest.mark.parametrize("nh, nkv, hd, page", [(16, 8, 128, 16), (8, 1, 64, 32), (4, 4, 64, 8), (12, 4, 128, 16),
                                                   (40, 2, 64, 16), (6, 3, 48, 16), (8, 2, 32, 8)])
