@@ -59,7 +59,7 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __g
   constexpr int KB_BYTES = TA_KEYS * 128;               // one [TA_KEYS][64] bfloat16 block of K or V
   constexpr uint32_t TMEM_COLS = TA_KEYS == 128 ? 512 : 256;   // two S buffers of TA_KEYS columns, then the O tile
   extern __shared__ unsigned char ta_smem_raw[];
-  __shared__ __align__(8) unsigned long long q_bar, k_full[2], k_empty[2], v_full[2], v_empty[2], s_ready[2], p_ready, p_free[2], o_ready;
+  __shared__ __align__(8) unsigned long long q_bar, k_full[2], k_empty[2], v_full[2], v_empty[2], s_ready[2], p_ready[2], p_free[2], o_ready[2];
   __shared__ uint32_t tmem_slot;
   __shared__ float l_other[TA_ROWS];
   __shared__ float m_half[2][TA_ROWS];                  // the two threads of a row tell each other their half's maximum
@@ -94,12 +94,15 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __g
       tma::mbar_init(&v_full[s], 1);
       tma::mbar_init(&v_empty[s], 1);
     }
-    tma::mbar_init(&s_ready[0], 1);
-    tma::mbar_init(&s_ready[1], 1);
-    tma::mbar_init(&p_ready, 8);                          // one arrival per softmax warp
-    tma::mbar_init(&p_free[0], 1);
-    tma::mbar_init(&p_free[1], 1);
-    tma::mbar_init(&o_ready, 1);
+    // Two barriers a kind, by the tile's parity.  A warp arrives on p_ready for tile it + 2 behind S(it + 2), whose product is issued after
+    // the wait for P(it), all eight arrivals: it cannot arrive twice in a phase.  A wait on o_ready for P V (it) stands behind S(it + 1),
+    // issued after P V (it - 1), so the phase before, P V (it - 2), is over; P V (it + 2) needs this warp's P, so none is passed over.
+    for (int i = 0; i < 2; ++i) {
+      tma::mbar_init(&s_ready[i], 1);
+      tma::mbar_init(&p_ready[i], 8);                     // one arrival per softmax warp
+      tma::mbar_init(&p_free[i], 1);
+      tma::mbar_init(&o_ready[i], 1);
+    }
     tma::mbar_fence_init();
     tma::prefetch_map(&q_map);
     tma::prefetch_map(&kv_map);
@@ -179,7 +182,7 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __g
           ok = issue_qk(it + 1);
           if (!ok) break;
         }
-        ok = tma::mbar_wait(&p_ready, it & 1);             // P(it) is in shared memory, O is rescaled if it had to be
+        ok = tma::mbar_wait(&p_ready[s], (it >> 1) & 1);   // P(it) is in shared memory, O is rescaled if it had to be
         if (ok) ok = tma::mbar_wait(&v_full[s], (it >> 1) & 1);
         if (!ok) break;
         tc5::fence_after_sync();
@@ -191,7 +194,7 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __g
           const uint64_t b_desc = tc5::smem_desc_mn_major_sw128(v_s + s * KV_BYTES + k * 2048, KB_BYTES);
           tc5::mma_f16(tmem_o, a_desc, b_desc, idesc_o, it > 0 || k > 0);     // O accumulates over the key tiles
         }
-        tc5::commit(&o_ready);                             // P V (it) and everything before it are done
+        tc5::commit(&o_ready[s]);                          // P V (it) and everything before it are done
         tc5::commit(&p_free[s]);
         tc5::commit(&v_empty[s]);
       }
@@ -270,7 +273,7 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __g
         }
         if (it > 0 && __any_sync(0xffffffffu, raise)) {
           // Rescale this thread's half of its row of O in tensor memory, after P V (it - 1) has finished.
-          ok = tma::mbar_wait(&o_ready, (it - 1) & 1);
+          ok = tma::mbar_wait(&o_ready[(it - 1) & 1], ((it - 1) >> 1) & 1);
           if (ok) {
             tc5::fence_after_sync();
             float v[OC];
@@ -313,7 +316,7 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __g
         tc5::fence_before_sync();
       }
       __syncwarp();
-      if (ok && lane == 0) mbar_arrive(&p_ready);            // ok is the same in all lanes of a warp here
+      if (ok && lane == 0) mbar_arrive(&p_ready[s]);         // ok is the same in all lanes of a warp here
     }
     // the row's sum is the two threads' sums; softmax warps meet at a named barrier of their own
     if (half == 1) l_other[r] = l;
@@ -324,7 +327,7 @@ attn_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap q_map, const __g
     asm volatile("bar.sync 1, 256;\n" ::: "memory");
     l = l_other[r];
     if (sink) l += ex2(-(m == neg_inf ? 0.f : m) * scale_log2);         // a key of score 0 that has no value
-    if (ok) ok = tma::mbar_wait(&o_ready, (n_tiles - 1) & 1);          // the last P V is done
+    if (ok) ok = tma::mbar_wait(&o_ready[(n_tiles - 1) & 1], ((n_tiles - 1) >> 1) & 1);          // the last P V is done
     float o_acc[OC];
     if (ok) {
       tc5::fence_after_sync();

@@ -615,7 +615,7 @@ def test_tcgen05_prefill_with_warps_that_drift_apart(ops, hd, apart):
     local = torch.cat([torch.arange(n, device=DEV) for n in ql])
     own = (local % 64 < 32)[:, None] & (torch.arange(nh, device=DEV) % 2 == 1)[None]
     q[:, :, 0] = torch.where(own == apart, 6.0, -6.0).to(torch.bfloat16) * hd ** 0.5
-    for which in ("tcgen05_128",):
+    for which in ("tcgen05", "tcgen05_128"):
         first, ref = run_attention(ops, b, torch.bfloat16, None, which)
         close(first, ref, torch.bfloat16)
         for _ in range(10):
