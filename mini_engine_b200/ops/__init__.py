@@ -1272,6 +1272,7 @@ def gla_chunk_count(meta) -> int:
 # ---- attention through a latent --------------------------------------------------------------------
 LATENT_TILE_Q = 16        # query tokens per block of csrc/latent_attention.cu
 use_latent_mma = True     # bfloat16 latent attention on the tensor cores (csrc/latent_attention_mma.cu); a switch for comparisons
+LATENT_TCGEN05_KEYS = 64  # keys a tile of csrc/latent_attention_tcgen05.cu
 use_latent_tcgen05 = True # ... and its portions of prompts on tcgen05 (csrc/latent_attention_tcgen05.cu)
 
 
@@ -1303,11 +1304,18 @@ def latent_prep(proj: torch.Tensor, offsets: dict, c_weight: torch.Tensor, eps: 
 
 def latent_tcgen05_heads_per_block(q_abs, q_rot, pool, page_size: int, meta, out, scale: float) -> int:
     """How many heads share a block of the tcgen05 kernel for portions of prompts; 0 where the mma.sync kernel runs: sizes and pages that
-    the former does not take, rows that a tensor map cannot name, a step without an error word."""
+    the former does not take, rows that a tensor map cannot name, a step without an error word, and steps whose longest context is one
+    key tile.  There the former's fixed part (tensor memory, tensor maps, the queries' way to shared memory) is longer than the latter's whole
+    walk: 16 heads, us, mma.sync / tcgen05, rows of 256 + 64 values: 1 prompt of 8 tokens 14.3 / 18.4, of 33 16.4 / 18.4, 128 of 33 59 / 70,
+    128 of 64 100 / 98; 128 + 32: 1 of 64 12.3 / 14.3, 128 of 8 14.3 / 16.4, but 32 of 64 25 / 18 (small latents: two blocks an SM, many
+    prompts fill it).  From 65 keys on the former is level (1 prompt of 80: 21 / 18.5, 16.4 / 16.4) or ahead."""
+    H, T, C = q_abs.shape
+    if meta.max_context_len <= LATENT_TCGEN05_KEYS and (C > 128 or T <= 1024):
+        return 0
     if not (use_latent_tcgen05 and scale > 0 and getattr(meta, "error_flag", None) is not None and pool.is_contiguous()
             and (q_abs.data_ptr() | q_rot.data_ptr() | pool.data_ptr() | out.data_ptr()) % 16 == 0):
         return 0
-    return (_lib or require_extension()).me_latent_attention_tcgen05_heads_per_block(q_abs.shape[0], q_abs.shape[2], q_rot.shape[2], page_size)
+    return (_lib or require_extension()).me_latent_attention_tcgen05_heads_per_block(H, C, q_rot.shape[2], page_size)
 
 
 def latent_attention(q_abs: torch.Tensor, q_rot: torch.Tensor, pool: torch.Tensor, page_size: int, block_tables: torch.Tensor,

@@ -128,3 +128,28 @@ def test_warps_that_rescale_at_every_tile_beside_warps_that_never_do(C, R, page,
             err = (first[h, t0:t0 + lens[b]].double() - p @ keys[:, :C]).abs()
             assert bool((err <= 2.0 ** -7 * (p @ keys[:, :C].abs()) + 1e-6).all()), f"request {b}, head {h}"
         t0 += lens[b]
+
+
+@pytest.mark.parametrize("C, R, lens, contexts, taken", [(256, 64, [40, 64], [40, 64], False), (256, 64, [40, 3], [40, 65], True), (256, 64, [64] * 17, [64] * 17, False),
+                                                         (128, 32, [64] * 16, [64] * 16, False), (128, 32, [64] * 16 + [2], [64] * 16 + [2], True)])
+def test_steps_of_one_key_tile(C, R, lens, contexts, taken):
+    """Steps whose longest context is one key tile keep the mma.sync kernel, of small latents up to 1,024 tokens; the neighbouring sizes do not."""
+    H, gen, ops, T = 4, g(C), _ops(), sum(lens)
+    meta = _meta(lens, contexts)
+    meta.error_flag = torch.zeros(4, dtype=torch.int32, device=DEV)
+    pages = -(-max(contexts) // 16)
+    table = torch.arange(pages * len(lens), dtype=torch.int32, device=DEV).view(len(lens), pages)
+    pool = (torch.randn(pages * 16 * len(lens), C + R, generator=gen) * 0.5).bfloat16().to(DEV)
+    q, qr = (torch.randn(H, T, C, generator=gen) * 0.4).bfloat16().to(DEV), (torch.randn(T, H, R, generator=gen) * 0.4).bfloat16().to(DEV)
+    sink, out = torch.randn(H, generator=gen).to(DEV), torch.full((H, T, C), float("nan"), dtype=torch.bfloat16, device=DEV)
+    meta.tile_lists[32] = _tiles(lens, 32)
+    assert (ops.latent_tcgen05_heads_per_block(q, qr, pool, 16, meta, out, 0.3) > 0) == taken
+    ops.latent_attention(q, qr, pool, 16, table, meta, sink, None, out, 0.3)
+    assert not meta.error_flag.any()
+    t = 0
+    for b, n in enumerate(lens):
+        for i in range(n):
+            p = contexts[b] - n + i
+            ref = _plain_rows_attention(q[:, t].cpu(), qr[t].cpu(), pool[table[b, 0] * 16:][:p + 1].cpu(), C, 0.3, sink.cpu(), p)
+            assert torch.allclose(out[:, t].cpu().double(), ref, atol=2e-2, rtol=2e-2), f"request {b}, place {p}"
+            t += 1
