@@ -55,7 +55,7 @@ __device__ __forceinline__ void store_row32(float* dst, const float (&v)[32], in
 // are), g * sigmoid(alpha * g) * (u + shift).  SiLU-and-multiply is {0, 1, 0}.
 struct GluParams {
   float limit = 0.f, alpha = 1.f, shift = 0.f;
-  int act = -1;      // without the gate (EPI 0): an element-wise activation of common.cuh on the results, by number (-1: none)
+  int act = -1;      // without the gate (EPI 0): an element-wise activation of common.cuh on the results, by number (-1: none; EPI 2: ACT_RELU2_ROUNDED)
 };
 __device__ __forceinline__ float gated(float g, float u, const GluParams& p) {
   if (p.limit > 0.f) {
@@ -84,7 +84,12 @@ __device__ __forceinline__ void write_rows(Load&& load, Fix&& fix, unsigned char
       load(c, g);
       tc5::wait_ld();
       fix(c, g);
-      if (glu.act >= 0) act_apply_all<TO>(g, glu.act);
+      if (EPI == 2) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) g[j] = act_apply<TO>(g[j], ACT_RELU2_ROUNDED);
+      } else if (glu.act >= 0) {
+        act_apply_all<TO>(g, glu.act);
+      }
     }
   };
   if (!vec) {
@@ -870,6 +875,7 @@ ME_API int me_gemm_tcgen05_persistent(const void* map_a, const void* map_w, void
 #define ME_TP_CASE(BN_)                                                                                  \
   if (bn == BN_) {                                                                                       \
     if (epi == 1) rc = launch_tp<BN_, 1, bf16>(map_a, map_w, C, ldc, M, N, K, err, stream, glu);         \
+    else if (glu.act == ACT_RELU2_ROUNDED) rc = launch_tp<BN_, 2, bf16>(map_a, map_w, C, ldc, M, N, K, err, stream); \
     else if (c_dtype == ME_BF16) rc = launch_tp<BN_, 0, bf16>(map_a, map_w, C, ldc, M, N, K, err, stream, glu); \
     else rc = launch_tp<BN_, 0, float>(map_a, map_w, C, ldc, M, N, K, err, stream);                      \
   }
@@ -933,6 +939,8 @@ ME_API int me_gemm_tcgen05(const void* map_a, const void* map_w, void* C, int c_
 #define ME_TG_CASE(BN_)                                                                                              \
   if (bn == BN_) {                                                                                                   \
     if (epi == 1) rc = launch_tg<BN_, 1, bf16, false>(map_a, map_w, C, ldc, M, N, K, 1, 0, err, stream, glu);        \
+    else if (glu.act == ACT_RELU2_ROUNDED) rc = deep ? launch_tg<BN_, 2, bf16, true>(map_a, map_w, C, ldc, M, N, K, 1, 0, err, stream)    \
+                                                     : launch_tg<BN_, 2, bf16, false>(map_a, map_w, C, ldc, M, N, K, 1, 0, err, stream);  \
     else if (c_dtype == ME_BF16) rc = deep ? launch_tg<BN_, 0, bf16, true>(map_a, map_w, C, ldc, M, N, K, 1, 0, err, stream, glu)   \
                                            : launch_tg<BN_, 0, bf16, false>(map_a, map_w, C, ldc, M, N, K, 1, 0, err, stream, glu); \
     else rc = deep ? launch_tg<BN_, 0, float, true>(map_a, map_w, C, ldc, M, N, K, splits, split_stride, err, stream)          \
@@ -961,6 +969,7 @@ ME_API int me_gemm_tcgen05_grouped(const void* map_a, const void* map_w, void* C
   GluParams gp;
   gp.limit = limit, gp.alpha = alpha, gp.shift = shift;
   gp.act = glu >= 2 ? glu - 2 : -1;
+  ME_REQUIRE(gp.act <= ACT_GELU_ERF, "me_gemm_tcgen05_grouped: activation %d", gp.act);
   ME_REQUIRE(bn == 128 || bn == 256, "me_gemm_tcgen05_grouped: tile width %d is not 128 or 256", bn);
 #define ME_GROUPED(BN_)                                                                                                          \
   if (glu == 1) rc = launch_grouped<BN_, 1, bf16>(map_a, map_w, C, ldc, offsets, E, rows, N, rows_w, K, gp, err, stream);        \
