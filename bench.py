@@ -813,7 +813,8 @@ def _logozen_roofline(cfg: dict, T: int, item: int, pk: dict, times: dict) -> di
     """What the design's own kernels have to move or do in a prefill step of T tokens, and the fraction of the measured
     peak that their summed time makes: bytes for the element-wise kernels, multiply-adds for attention and recurrence."""
     W, S = cfg["width"], cfg["streams"]
-    need = {"me_hc_norm": 0.0, "me_short_conv": 0.0, "me_polynorm": 0.0, "me_latent_attention_mma": 0.0, "me_mlstm_scan": 0.0}
+    need = {"me_hc_norm": 0.0, "me_short_conv": 0.0, "me_polynorm": 0.0, "me_latent_attention_mma": 0.0, "me_latent_attention_tcgen05": 0.0,
+            "me_mlstm_scan": 0.0}
     for layer in cfg["layers"]:
         m = layer["mixer"]
         subs = 2 if layer["mlp"] is not None else 1
@@ -822,11 +823,12 @@ def _logozen_roofline(cfg: dict, T: int, item: int, pk: dict, times: dict) -> di
         if layer["mlp"] is not None:
             need["me_polynorm"] += T * layer["mlp"]["ff"] * (4 + item)
         if layer["type"] == "latent_attention":
-            need["me_latent_attention_mma"] += 2.0 * m["heads"] * (2 * m["kv_rank"] + m["rot_dim"]) * T * (T + 1) / 2
+            for kernel in ("me_latent_attention_mma", "me_latent_attention_tcgen05"):      # whichever the size runs
+                need[kernel] += 2.0 * m["heads"] * (2 * m["kv_rank"] + m["rot_dim"]) * T * (T + 1) / 2
         else:
             need["me_mlstm_scan"] += 4.0 * m["heads"] * m["dim"] * m["vdim"] * T
     need["me_hc_norm"] += W * (4 * S + item)                               # the last norm, one row
-    return _fractions(need, ("me_latent_attention_mma", "me_mlstm_scan"), times, pk)
+    return _fractions(need, ("me_latent_attention_mma", "me_latent_attention_tcgen05", "me_mlstm_scan"), times, pk)
 
 
 def _fractions(need: dict, flop_kernels, times: dict, pk: dict) -> dict:
@@ -933,7 +935,7 @@ def _galupel_roofline(cfg: dict, T: int, item: int, pk: dict, times: dict) -> di
     their summed time makes: bytes for the element-wise kernels, multiply-adds for attention and experts."""
     W = cfg["width"]
     need = {k: 0.0 for k in ("me_group_norm", "me_attn_prep", "me_pool_kv", "me_sink_attn", "me_attn_prefill_tcgen05", "me_latent_prep",
-                             "me_latent_attention_mma", "me_moe_gemm", "me_gemm_tcgen05_grouped", "me_activation", "me_moe_combine")}
+                             "me_latent_attention_mma", "me_latent_attention_tcgen05", "me_moe_gemm", "me_gemm_tcgen05_grouped", "me_activation", "me_moe_combine")}
     need["me_group_norm"] += T * W * (8 + item) + W * (4 + item)            # behind the embedding, and the last norm's one row
     for layer in cfg["layers"]:
         m, mlp = layer["mixer"], layer["mlp"]
@@ -954,14 +956,15 @@ def _galupel_roofline(cfg: dict, T: int, item: int, pk: dict, times: dict) -> di
         else:
             C, R = m["kv_rank"], m["rot_dim"]
             need["me_latent_prep"] += T * ((H * (m["dim"] + R) + C + R) * 4 + (H * (m["dim"] + R) + C + R) * item)
-            need["me_latent_attention_mma"] += 2.0 * H * (2 * C + R) * _window_pairs(T, size)
+            for kernel in ("me_latent_attention_mma", "me_latent_attention_tcgen05"):      # whichever the size runs
+                need[kernel] += 2.0 * H * (2 * C + R) * _window_pairs(T, size)
         if mlp is not None:
             pairs, F = T * mlp["router"]["top"], mlp["expert"]["ff"]
             need["me_moe_gemm"] += 4.0 * pairs * F * W
             need["me_gemm_tcgen05_grouped"] += 4.0 * pairs * F * W
             need["me_activation"] += pairs * F * 2 * item
             need["me_moe_combine"] += T * W * (4 * mlp["router"]["top"] + 4)
-    return _fractions(need, ("me_sink_attn", "me_attn_prefill_tcgen05", "me_latent_attention_mma", "me_moe_gemm", "me_gemm_tcgen05_grouped"),
+    return _fractions(need, ("me_sink_attn", "me_attn_prefill_tcgen05", "me_latent_attention_mma", "me_latent_attention_tcgen05", "me_moe_gemm", "me_gemm_tcgen05_grouped"),
                       times, pk)
 
 
