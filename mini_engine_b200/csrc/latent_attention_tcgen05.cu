@@ -8,13 +8,14 @@
 //     O[128 x C] += P V with P from tensor memory and V as an MN-major operand from K's own tile.  O stays in tensor memory.
 //   warps 2..5: bring Q once, then a thread a row: scores from tensor memory, mask, maximum, exponentials; P (bfloat16, two a column)
 //     goes over the S buffer it came from.  Where a row's maximum rises its row of O is rescaled in tensor memory.  At the end O leaves through Q's place in shared memory in whole rows.
-// What bounds it: the products.  Of a tile of 256 + 64 columns Q K^T reads 120 KB of shared memory (20 products of N = 64, a little more
-// than they take to multiply), P V 32 KB; the softmax of the tile, some 1,000 clocks of latency in four warps, runs beside the next tile's
-// Q K^T.  Q, 80 KB, and three tiles of 40 KB take the SM; rows of up to 192 values and latents of up to 128 leave room for two blocks
-// with two tiles each, which then wait for their loads in turn.
-// Measured beside the mma.sync kernel (one B200, 3 prompts of 400, 800 and 1,250 tokens, 16 heads; with the reference raised by steps of
-// more than 2^8 only, before it followed the maximum): rows of 256 + 64 values 194 -> 54 us, 128 + 32 95 -> 45, 64 + 8 79 -> 37; one prompt
-// of 4,000 tokens 1,031 -> 179, of 300 44 -> 18, of 64 level on the device.
+// What bounds it: a tile's chain of waits, not the products (tensor pipe 22% of the active clocks at 256 + 64 values, 17% at 128 + 32).  Four
+// warps read a row of S, reduce it, rescale O where the maximum rose, form and store P, and P V follows; only the next tile's Q K^T runs
+// beside that: 1.5 us a tile with three tiles in the ring, 2.1 with two, where a load also waits for the P V two tiles before.  Q, 80 KB at
+// 256 + 64, and three tiles of 40 KB take the SM; rows of up to 192 values and latents of up to 128 leave room for two blocks with two
+// tiles each, which fill one another's waits.  Blocks are uneven (the last tokens of a prompt see all its keys): the rest of the time.
+// Measured beside the mma.sync kernel (one B200, L2 flushed, 16 heads, us): 3 prompts of 400, 800 and 1,250 tokens, rows of 256 + 64 values
+// 199 -> 61, 192 + 64 123 -> 54, 128 + 32 104 -> 53, 64 + 8 87 -> 47; one prompt of 4,000 tokens 1,038 -> 203 (256 + 64), 371 -> 170 (128 + 32),
+// of 300 47 -> 25, 27 -> 22; 16 tokens behind 4,000 485 -> 109, 211 -> 144.  Steps of one key tile stay with that kernel (ops).
 // All waits are bounded; a wait that gives up sets flag 1 of ``err`` and the block frees its tensor memory and exits.
 #include "tcgen05.cuh"
 #include "mma_prims.cuh"

@@ -58,7 +58,8 @@ def test_portions_of_prompts(H, C, R, page, lens, contexts, window):
             ref = _plain_rows_attention(qa[t], qr[t], rows[b][lo:], C, 0.3, sink, p - lo) * gate[t].double()[:, None]
             assert torch.allclose(got[t], ref, atol=2e-2, rtol=2e-2), f"request {b}, place {p}"
             err, err_old, t = err + float((got[t] - ref).square().sum()), err_old + float((old[t] - ref).square().sum()), t + 1
-    assert err <= 1.1 * err_old                               # the same roundings: no further from 64 bits
+    # the same roundings: level with the other kernel (0.970 to 1.006 of its sum of squares over these cases; larger batches, 12 seeds: 0.98 to 1.00)
+    assert err <= 1.02 * err_old
 
 
 def test_infinite_scores_and_rows_beside_them():
